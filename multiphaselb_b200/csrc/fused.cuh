@@ -289,7 +289,7 @@ __device__ __forceinline__ void pull_node(const Params& P, const FusedArgs& A, i
 // Interaction force, total force and velocity of one node from its
 // post-stream populations f, density rho (rr = RN(1/rho)) and psi
 // (nbpsi(k) = psi_n at x + c_k).
-template <class L, class PsiAt>
+template <class L, bool EMIT, class PsiAt>
 __device__ __forceinline__ void force_velocity(const Params& P, bool onb, const double* f, double rho, double rr,
                                                double psi, PsiAt nbpsi, double* Fi, double* Ft, double* U) {
     Fi[0] = Fi[1] = Fi[2] = 0;
@@ -309,31 +309,49 @@ __device__ __forceinline__ void force_velocity(const Params& P, bool onb, const 
 #pragma unroll
         for (int i = 0; i < 3; i++) Fi[i] = F[i] * be;
     }
-    // interForce.c:27-39
+    // interForce.c:27-39.  Without body force Ft is Fi (plus zeros, which change
+    // no value); the rebuild of the reference state (EMIT) adds them all the same.
+    if (EMIT || P.body) {
 #pragma unroll
-    for (int j = 0; j < 3; j++) {
-        double t = Fi[j] + (rho - P.rho_0) * P.g[j];
-        if (!onb) t += P.fext[j];
-        Ft[j] = t;
+        for (int j = 0; j < 3; j++) {
+            double t = Fi[j] + (rho - P.rho_0) * P.g[j];
+            if (!onb) t += P.fext[j];
+            Ft[j] = t;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 3; j++) Ft[j] = Fi[j];
     }
     // liMRTVelocity.c:27-44 (F = Ft) / xuMRTVelocity.c:19-44 (F = Fi + (rho - rho_0) g).
     // Zero velocity components contribute +-0 and are skipped.
+    // In 2D the third component is zero unless a body force acts along it.
     static_for<3>([&](auto jj) {
         constexpr int j = decltype(jj)::value;
+        if (!EMIT && L::D == 2 && j == 2 && !P.body_z) {
+            U[j] = 0;
+            return;
+        }
         double lv = 0;
         static_for<L::Q>([&](auto kk) {
             constexpr int c = ck<L>(decltype(kk)::value, j);
             if constexpr (c == 1) lv = lv + f[kk];
             else if constexpr (c == -1) lv = lv - f[kk];
         });
-        double Fj = L::Q == 9 ? Ft[j] : Fi[j] + (rho - P.rho_0) * P.g[j];
+        double Fj = L::Q == 9 ? Ft[j] : (EMIT || P.body ? Fi[j] + (rho - P.rho_0) * P.g[j] : Fi[j]);
         U[j] = div_rcp(lv + Fj * 0.5, rho, rr);  // == (lv + Fj*0.5)/rho
     });
 }
 
 // Everything after the macros for one node that owns an output.
-// nbpsi(k) returns psi_n at x + c_k.
-template <class L, bool F_ON, bool G_ON, bool EMIT, class PsiAt, bool MY = false>
+// nbpsi(k) returns psi_n at x + c_k.  ST: the flow has a surface-tension term.
+// It is a kernel variant of its own: a step is bound by FP64 issue and latency
+// (about 530 FP64 instructions a node), and the term's moments, although not
+// evaluated, cost every kernel registers and spills inside its plane or tile
+// loop.  Without them, and without the operations whose value is known
+// (moment 0, zero body forces, the zero test in div_rcp), the D3Q15 step on a
+// periodic 192^3 went from 546 to 480 us, the thermal 1024 x 4096 column from
+// 340 to 325 us, the 256^2 bubble from 4.36 to 4.06 us (B200, back to back).
+template <class L, bool F_ON, bool G_ON, bool EMIT, class PsiAt, bool MY = false, bool ST = false>
 __device__ __forceinline__ void finish_node(const Params& P, const FusedArgs& A, uint32_t id, bool onb,
                                             double* f, double* g, double rho, double rr, double T, double psi,
                                             PsiAt nbpsi, double src_heat) {
@@ -343,7 +361,7 @@ __device__ __forceinline__ void finish_node(const Params& P, const FusedArgs& A,
         if (id - A.own_lo >= A.own_cnt) return;
     double Fi[3] = {0, 0, 0}, Ft[3], U[3];
     if constexpr (F_ON) {
-        force_velocity<L>(P, onb, f, rho, rr, psi, nbpsi, Fi, Ft, U);
+        force_velocity<L, EMIT>(P, onb, f, rho, rr, psi, nbpsi, Fi, Ft, U);
     } else {
 #pragma unroll
         for (int j = 0; j < 3; j++) U[j] = A.Uold[(size_t)j * n + id];
@@ -368,19 +386,18 @@ __device__ __forceinline__ void finish_node(const Params& P, const FusedArgs& A,
     }
     if constexpr (F_ON) {
         // surface-tension term (zero on wall nodes, which miss a neighbour)
-        double C[L::Q];
-        const double* Cp = nullptr;
-        if (P.st_on) {
-            if (!onb) {
-                surface_tension<L>(P, psi, nbpsi, C);
-            } else {
+        auto term = [&](double* m) {
+            if constexpr (ST) {
+                if (!onb) {
+                    double C[L::Q];
+                    surface_tension<L>(P, psi, nbpsi, C);
 #pragma unroll
-                for (int k = 0; k < L::Q; k++) C[k] = 0;
+                    for (int k = 0; k < L::Q; k++) m[k] = m[k] + C[k];
+                }
             }
-            Cp = C;
-        }
-        if constexpr (L::Q == 9) collide_limrt_psi(P, f, rho, U, Ft, Fi, psi, Cp);
-        else collide_xumrt_psi(P, f, rho, U, Fi, psi, Cp);
+        };
+        if constexpr (L::Q == 9) collide_limrt_psi<true>(P, f, rho, U, Ft, Fi, psi, term);
+        else collide_xumrt_psi<true>(P, f, rho, U, Fi, psi, term);
 #pragma unroll
         for (int k = 0; k < L::Q; k++) A.fout[(size_t)k * n + id] = f[k];
         if constexpr (G_ON) {
@@ -391,7 +408,7 @@ __device__ __forceinline__ void finish_node(const Params& P, const FusedArgs& A,
     }
     if constexpr (G_ON) {
         if constexpr (MY) collide_mymrt<L>(P, g, T, U, src_heat);
-        else collide_litemp(P, g, T, U[0], U[1], src_heat);
+        else collide_litemp<true>(P, g, T, U[0], U[1], src_heat);
 #pragma unroll
         for (int k = 0; k < 9; k++) A.gout[(size_t)k * n + id] = g[k];
         A.Tnew[id] = T;
@@ -521,7 +538,7 @@ __global__ void __launch_bounds__(256) k_pullsum_d2q9(Params P, FusedArgs A) {
 // tiles skip the wrap / missing-source / boundary bookkeeping; the
 // arithmetic is the same code either way.
 template <int F2_TX, int F2_TY, bool F_ON, bool G_ON, bool HAS_BC, bool EMIT, bool INNER, int EX, int EY, int GX,
-          int GY, bool MY = false, int RINGW = 0>
+          int GY, bool MY = false, int RINGW = 0, bool ST = false>
 __device__ __forceinline__ void fused2_tile(const Params& P, const FusedArgs& A, int x0, int y0,
                                             double (*s_psi)[EX], double (*s_inv)[GX], double (*s_To)[GX],
                                             double (*s_U0)[GX], double (*s_U1)[GX]) {
@@ -661,7 +678,7 @@ __device__ __forceinline__ void fused2_tile(const Params& P, const FusedArgs& A,
     double psi = 0;
     if constexpr (F_ON) psi = s_psi[ey][ex];
     auto nbpsi = [&](int k) { return s_psi[ey + cyk<L>(k)][ex + cxk<L>(k)]; };
-    finish_node<L, F_ON, G_ON, EMIT, decltype(nbpsi), MY>(P, A, id, onb, f, g, rho, rr, T, psi, nbpsi, heat);
+    finish_node<L, F_ON, G_ON, EMIT, decltype(nbpsi), MY, ST>(P, A, id, onb, f, g, rho, rr, T, psi, nbpsi, heat);
 }
 
 // MINB: resident blocks per SM asked of the register allocator (0 = the
@@ -674,7 +691,7 @@ __device__ __forceinline__ void fused2_tile(const Params& P, const FusedArgs& A,
 // RINGW: warps added to the block that compute the tile's ring (launch with
 // TX * TY + 32 * RINGW threads); 0: the node threads compute it first.
 template <int F2_TX, int F2_TY, int MINB, bool F_ON, bool G_ON, bool HAS_BC, bool EMIT, bool TRY_INNER = false,
-          bool MY = false, int RINGW = 0>
+          bool MY = false, int RINGW = 0, bool ST = false>
 __global__ void __launch_bounds__(F2_TX * F2_TY + 32 * RINGW, MINB ? MINB : min_blocks(F2_TX * F2_TY))
     k_fused_d2q9(Params P, FusedArgs A) {
     step_dependency_wait();
@@ -689,13 +706,13 @@ __global__ void __launch_bounds__(F2_TX * F2_TY + 32 * RINGW, MINB ? MINB : min_
     const int x0 = bx * F2_TX, y0 = by * F2_TY;
     if constexpr (TRY_INNER) {
         if (inner_tile<F2_TX, F2_TY>(A, x0, y0)) {
-            fused2_tile<F2_TX, F2_TY, F_ON, G_ON, HAS_BC, EMIT, true, EX, EY, GX, GY, MY, RINGW>(
+            fused2_tile<F2_TX, F2_TY, F_ON, G_ON, HAS_BC, EMIT, true, EX, EY, GX, GY, MY, RINGW, ST>(
                 P, A, x0, y0, s_psi, s_inv, s_To, s_U0, s_U1);
             return;
         }
     }
-    fused2_tile<F2_TX, F2_TY, F_ON, G_ON, HAS_BC, EMIT, false, EX, EY, GX, GY, MY, RINGW>(P, A, x0, y0, s_psi, s_inv,
-                                                                                          s_To, s_U0, s_U1);
+    fused2_tile<F2_TX, F2_TY, F_ON, G_ON, HAS_BC, EMIT, false, EX, EY, GX, GY, MY, RINGW, ST>(
+        P, A, x0, y0, s_psi, s_inv, s_To, s_U0, s_U1);
 }
 
 // ------------------------------------------------------------ 3D kernels
@@ -710,7 +727,7 @@ constexpr size_t f3_smem() {
     return (size_t)(3 * (TY + 2) * (TX + 2) + (PIPE ? 3 : 2) * 15 * TX * TY) * sizeof(double);
 }
 
-template <int F3_TX, int F3_TY, bool HAS_BC, bool EMIT>
+template <int F3_TX, int F3_TY, bool HAS_BC, bool EMIT, bool ST = false>
 __global__ void __launch_bounds__(F3_TX * F3_TY, min_blocks(F3_TX * F3_TY)) k_fused_d3q15(Params P, FusedArgs A) {
     step_dependency_wait();
     using L = D3Q15T;
@@ -776,7 +793,8 @@ __global__ void __launch_bounds__(F3_TX * F3_TY, min_blocks(F3_TX * F3_TY)) k_fu
             auto nbpsi = [&](int k) {
                 return s_psi[(z + czk<L>(k) + 3) % 3][ey + cyk<L>(k)][ex + cxk<L>(k)];
             };
-            finish_node<L, true, false, EMIT>(P, A, idc, onb, f, dum, rc, rrc, Tc, s_psi[z % 3][ey][ex], nbpsi, 0.0);
+            finish_node<L, true, false, EMIT, decltype(nbpsi), false, ST>(P, A, idc, onb, f, dum, rc, rrc, Tc,
+                                                                          s_psi[z % 3][ey][ex], nbpsi, 0.0);
         }
         __syncthreads();
         rc = rn;

@@ -91,13 +91,13 @@ inline const TmaMaps* tma_maps(FusedConfig& fc, int cfg, const FusedArgs& A, uin
     return &m;
 }
 
-template <int TX, int TY, bool PIPE, bool HAS_BC, bool EMIT>
+template <int TX, int TY, bool PIPE, bool HAS_BC, bool EMIT, bool ST = false>
 cudaError_t set_smem3() {
     if constexpr (PIPE)
         return cudaFuncSetAttribute(k_fused_d3q15_pipe<TX, TY, HAS_BC, EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)f3_smem<TX, TY, PIPE>());
     else
-        return cudaFuncSetAttribute(k_fused_d3q15<TX, TY, HAS_BC, EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        return cudaFuncSetAttribute(k_fused_d3q15<TX, TY, HAS_BC, EMIT, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)f3_smem<TX, TY, PIPE>());
 }
 
@@ -107,6 +107,8 @@ inline cudaError_t fused_attributes() {
     auto chk = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     chk(set_smem3<32, 8, false, true, true>());
     chk(set_smem3<32, 8, false, false, true>());
+    chk(set_smem3<32, 8, false, true, false, true>());
+    chk(set_smem3<32, 8, false, false, false, true>());
 #define MPLB_SET3(TX, TY, PIPE) chk(set_smem3<TX, TY, PIPE, true, false>()); chk(set_smem3<TX, TY, PIPE, false, false>());
     MPLB_SET3(32, 8, false)
     MPLB_SET3(32, 8, true)
@@ -115,14 +117,16 @@ inline cudaError_t fused_attributes() {
     MPLB_SET3(32, 16, false)
     MPLB_SET3(64, 8, false)
 #undef MPLB_SET3
-    chk(cudaFuncSetAttribute(k_fused_d3q15_tma<32, 4, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)TmaTile<32, 4>::SMEM));
-    chk(cudaFuncSetAttribute(k_fused_d3q15_tma<32, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)TmaTile<32, 8>::SMEM));
-    chk(cudaFuncSetAttribute(k_fused_d3q15_tma<32, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)TmaTile<32, 16>::SMEM));
-    chk(cudaFuncSetAttribute(k_fused_d3q15_tma<64, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)TmaTile<64, 8>::SMEM));
+#define MPLB_SET3_TMA(TX, TY, MINB)                                                                                          \
+    chk(cudaFuncSetAttribute(k_fused_d3q15_tma<TX, TY, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
+                             (int)TmaTile<TX, TY>::SMEM));                                                                  \
+    chk(cudaFuncSetAttribute(k_fused_d3q15_tma<TX, TY, MINB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
+                             (int)TmaTile<TX, TY>::SMEM));
+    MPLB_SET3_TMA(32, 4, 3)
+    MPLB_SET3_TMA(32, 8, 2)
+    MPLB_SET3_TMA(32, 16, 1)
+    MPLB_SET3_TMA(64, 8, 1)
+#undef MPLB_SET3_TMA
     return e;
 }
 
@@ -130,15 +134,17 @@ template <int TX, int TY, int MINB>
 cudaError_t launch3_tma(FusedConfig& fc, int cfg, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
     const TmaMaps* m = tma_maps(fc, cfg, A, P.n);
     if (!m) return cudaErrorInvalidValue;
-    launch_step(k_fused_d3q15_tma<TX, TY, MINB>, nb, TX * TY, TmaTile<TX, TY>::SMEM, s, P, A, m->mf, m->mT);
+    if (P.st_on) launch_step(k_fused_d3q15_tma<TX, TY, MINB, true>, nb, TX * TY, TmaTile<TX, TY>::SMEM, s, P, A, m->mf, m->mT);
+    else launch_step(k_fused_d3q15_tma<TX, TY, MINB>, nb, TX * TY, TmaTile<TX, TY>::SMEM, s, P, A, m->mf, m->mT);
     return cudaSuccess;
 }
 
-template <int TX, int TY, int MINB, bool F_ON, bool G_ON, bool EMIT, bool INNER, bool MY = false, int RINGW = 0>
+template <int TX, int TY, int MINB, bool F_ON, bool G_ON, bool EMIT, bool INNER, bool MY = false, int RINGW = 0,
+          bool ST = false>
 void launch2(bool bc, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
     constexpr int nt = TX * TY + 32 * RINGW;
-    if (bc) launch_step(k_fused_d2q9<TX, TY, MINB, F_ON, G_ON, true, EMIT, INNER, MY, RINGW>, nb, nt, 0, s, P, A);
-    else launch_step(k_fused_d2q9<TX, TY, MINB, F_ON, G_ON, false, EMIT, INNER, MY, RINGW>, nb, nt, 0, s, P, A);
+    if (bc) launch_step(k_fused_d2q9<TX, TY, MINB, F_ON, G_ON, true, EMIT, INNER, MY, RINGW, ST>, nb, nt, 0, s, P, A);
+    else launch_step(k_fused_d2q9<TX, TY, MINB, F_ON, G_ON, false, EMIT, INNER, MY, RINGW, ST>, nb, nt, 0, s, P, A);
 }
 
 // myMRT steps first fill rho_a, gsum_a (k_pullsum_d2q9).
@@ -149,7 +155,7 @@ void launch_pullsum(bool bc, const Params& P, const FusedArgs& A, cudaStream_t s
     else launch_step(k_pullsum_d2q9<F_ON, false>, nb, 256, 0, s, P, A);
 }
 
-template <int TX, int TY, bool EMIT, int MINB = 0, bool INNER = false, int RINGW = 0>
+template <int TX, int TY, bool EMIT, int MINB = 0, bool INNER = false, int RINGW = 0, bool ST = false>
 void launch2_fg(bool fon, bool gon, bool bc, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
     const bool my = gon && P.g_model == MPLB_MYMRT;
     if (my) {
@@ -157,38 +163,43 @@ void launch2_fg(bool fon, bool gon, bool bc, int nb, const Params& P, const Fuse
             if (fon) launch_pullsum<true>(bc, P, A, s);
             else launch_pullsum<false>(bc, P, A, s);
         }
-        if (fon) launch2<TX, TY, MINB, true, true, EMIT, INNER, true, RINGW>(bc, nb, P, A, s);
-        else launch2<TX, TY, MINB, false, true, EMIT, INNER, true, RINGW>(bc, nb, P, A, s);
+        if (fon) launch2<TX, TY, MINB, true, true, EMIT, INNER, true, RINGW, ST>(bc, nb, P, A, s);
+        else launch2<TX, TY, MINB, false, true, EMIT, INNER, true, RINGW, false>(bc, nb, P, A, s);
         return;
     }
-    if (fon && gon) launch2<TX, TY, MINB, true, true, EMIT, INNER, false, RINGW>(bc, nb, P, A, s);
-    else if (fon) launch2<TX, TY, MINB, true, false, EMIT, INNER, false, RINGW>(bc, nb, P, A, s);
-    else if (gon) launch2<TX, TY, MINB, false, true, EMIT, INNER, false, RINGW>(bc, nb, P, A, s);
+    if (fon && gon) launch2<TX, TY, MINB, true, true, EMIT, INNER, false, RINGW, ST>(bc, nb, P, A, s);
+    else if (fon) launch2<TX, TY, MINB, true, false, EMIT, INNER, false, RINGW, ST>(bc, nb, P, A, s);
+    else if (gon) launch2<TX, TY, MINB, false, true, EMIT, INNER, false, RINGW, false>(bc, nb, P, A, s);
 }
 
-template <int TX, int TY, bool PIPE, bool EMIT>
+template <int TX, int TY, bool PIPE, bool EMIT, bool ST = false>
 void launch3(bool bc, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
     constexpr size_t sm = f3_smem<TX, TY, PIPE>();
     if constexpr (PIPE) {
         if (bc) launch_step(k_fused_d3q15_pipe<TX, TY, true, EMIT>, nb, TX * TY, sm, s, P, A);
         else launch_step(k_fused_d3q15_pipe<TX, TY, false, EMIT>, nb, TX * TY, sm, s, P, A);
     } else {
-        if (bc) launch_step(k_fused_d3q15<TX, TY, true, EMIT>, nb, TX * TY, sm, s, P, A);
-        else launch_step(k_fused_d3q15<TX, TY, false, EMIT>, nb, TX * TY, sm, s, P, A);
+        if (bc) launch_step(k_fused_d3q15<TX, TY, true, EMIT, ST>, nb, TX * TY, sm, s, P, A);
+        else launch_step(k_fused_d3q15<TX, TY, false, EMIT, ST>, nb, TX * TY, sm, s, P, A);
     }
 }
 
 // Launch one fused step with candidate `cfg` (EMIT always uses candidate 0).
 inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, FusedArgs A, bool f_on, bool g_on,
                                     bool emit, cudaStream_t s) {
-    if (emit) cfg = 0;
+    // surface tension: one tile shape per kernel family stands for all candidates
+    const bool st = P.st_on && f_on && !emit;
+    const bool tma = fc.lat == MPLB_D3Q15 && CFG3[cfg].tma;
+    if (fc.geom[cfg].nblocks == 0 && !emit) return cudaErrorInvalidConfiguration;  // the candidate does not take this lattice
+    if (emit || (st && !tma)) cfg = 0;
     apply_geom(A, fc.geom[cfg]);
     const int nb = fc.geom[cfg].nblocks;
-    if (nb == 0) return cudaErrorInvalidConfiguration;  // the candidate does not take this lattice
     const bool bc = fc.has_bc;
     if (fc.lat == MPLB_D2Q9) {
         if (emit) {
             launch2_fg<32, 8, true>(f_on, g_on, bc, nb, P, A, s);
+        } else if (st) {
+            launch2_fg<32, 8, false, 0, false, 0, true>(f_on, g_on, bc, nb, P, A, s);
         } else {
             switch (cfg) {
             case 0: launch2_fg<32, 8, false>(f_on, g_on, bc, nb, P, A, s); break;
@@ -206,6 +217,8 @@ inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, F
     } else {
         if (emit) {
             launch3<32, 8, false, true>(bc, nb, P, A, s);
+        } else if (st && !tma) {
+            launch3<32, 8, false, false, true>(bc, nb, P, A, s);
         } else {
             switch (cfg) {
             case 0: launch3<32, 8, false, false>(bc, nb, P, A, s); break;

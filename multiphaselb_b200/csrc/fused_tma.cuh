@@ -60,7 +60,7 @@ struct TmaTile {
     static_assert(TX % 2 == 0, "x0 - 2 must be even");
 };
 
-template <int TX, int TY, int MINB>
+template <int TX, int TY, int MINB, bool ST = false>
 __global__ void __launch_bounds__(TX * TY, MINB)
     k_fused_d3q15_tma(Params P, FusedArgs A, const __grid_constant__ CUtensorMap tm_f,
                       const __grid_constant__ CUtensorMap tm_T) {
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(TX * TY, MINB)
                 return s_psi[(z + czk<L>(k) + G::NPSI) % G::NPSI][ey + cyk<L>(k)][ex + cxk<L>(k)];
             };
             double dum[1];
-            finish_node<L, true, false, false>(P, A, id, false, fp, dum, rp, rrp, Tp,
+            finish_node<L, true, false, false, decltype(nbpsi), false, ST>(P, A, id, false, fp, dum, rp, rrp, Tp,
                                                s_psi[(z + G::NPSI) % G::NPSI][ey][ex], nbpsi, 0.0);
         }
 #pragma unroll

@@ -103,6 +103,8 @@ struct Params {
     // exact shortcuts, decided on the host: x/G == -x when G == -1,
     // x/Cv == x when Cv == 1, x/(M*M) == x when M*M == 1
     int32_t g_neg1, cv_one, m2_one;
+    int32_t body;    // any of g, fext is non-zero
+    int32_t body_z;  // any of g[2], fext[2] is non-zero
     // surface-tension term of the flow field (liMRT/xuMRT surfaceTension, kappa_st)
     int32_t st_on;
     double kappa_st;
@@ -115,11 +117,15 @@ struct Params {
 // e = x - q*y is exact in one FMA and RN(q + e*yr) = RN(x/y), for results
 // that neither overflow nor underflow.  So several quotients with the same
 // divisor cost one reciprocal and three operations each, and are bit-equal to
-// IEEE division.  A zero numerator returns q, which keeps the sign of x/y.
+// IEEE division, but for x = -0, which gives +0 (RN(q + e*yr) of q = -0,
+// e = +0).  No numerator on the path is -0 where the sign of a zero quotient
+// could be seen: the velocity's is a sum that starts from +0, the EOS's are
+// positive, and a zero equilibrium or source moment is only added to or
+// subtracted from a moment that is itself a sum from +0, hence never -0.
 MPLB_HD double div_rcp(double x, double y, double yr) {
     const double q = x * yr;
     const double e = fma(-q, y, x);
-    return q == 0.0 ? q : fma(e, yr, q);
+    return fma(e, yr, q);
 }
 // RN(1/3) for x/3.0.
 constexpr double RCP3 = 1.0 / 3.0;
@@ -240,12 +246,14 @@ MPLB_HD double add_exact_product(double s, double c, double v) {
 #endif
 }
 
-template <class L>
+// FIRST: the first row to evaluate (row 0, the sum, may be known already).
+template <class L, int FIRST = 0>
 MPLB_HD void mul_M(const double* v, double* r) {
-    static_for<L::Q>([&](auto i) {
+    static_for<L::Q - FIRST>([&](auto im) {
+        constexpr int i = decltype(im)::value + FIRST;
         double s = 0;
         static_for<L::Q>([&](auto j) {
-            constexpr int c = Mint<L>(decltype(i)::value, decltype(j)::value);
+            constexpr int c = Mint<L>(i, decltype(j)::value);
             if constexpr (c == 1) s = s + v[j];
             else if constexpr (c == -1) s = s - v[j];
             else if constexpr (pow2_ge2(c)) s = add_exact_product(s, (double)c, v[j]);
@@ -370,10 +378,18 @@ MPLB_HD void surface_tension(const Params& P, double ps, PsiAt nbpsi, double* C)
     }
 }
 
-// C (may be NULL) is the surface-tension term, added to every moment after
-// the relaxation (liMRTCollision.c:90-98).
+// No term after the relaxation.
+struct NoTerm {
+    MPLB_HD void operator()(double*) const {}
+};
+
+// term(m) adds the surface-tension moments after the relaxation
+// (liMRTCollision.c:90-98).  SUM0: rho is the sum of f in k order (the fused
+// steps), so moment 0 is rho itself and, with its equilibrium equal to it and
+// no source, stays so: rho - L0 * 0 + r0 * 0.
+template <bool SUM0 = false, class Term = NoTerm>
 MPLB_HD void collide_limrt_psi(const Params& P, double* f, double rho, const double* U,
-                               const double* F, const double* Fi, double ps, const double* C = nullptr) {
+                               const double* F, const double* Fi, double ps, Term term = Term()) {
     double um = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) um += U[k] * U[k];
@@ -387,7 +403,8 @@ MPLB_HD void collide_limrt_psi(const Params& P, double* f, double rho, const dou
     meq[6] = rho * (-U[1]);
     meq[7] = rho * (U[0] * U[0] - U[1] * U[1]);
     meq[8] = rho * U[0] * U[1];
-    mul_M<D2Q9T>(f, m);
+    mul_M<D2Q9T, SUM0 ? 1 : 0>(f, m);
+    if (SUM0) m[0] = rho;
     double uf = U[0] * F[0] + U[1] * F[1];
     double fi2 = Fi[0] * Fi[0] + Fi[1] * Fi[1];
     S[0] = 0;
@@ -400,11 +417,8 @@ MPLB_HD void collide_limrt_psi(const Params& P, double* f, double rho, const dou
     S[7] = 2 * (U[0] * F[0] - U[1] * F[1]);
     S[8] = U[0] * F[1] + U[1] * F[0];
 #pragma unroll
-    for (int k = 0; k < 9; k++) m[k] = m[k] - P.Lf[k] * (m[k] - meq[k]) + P.relax_f[k] * S[k];
-    if (C) {
-#pragma unroll
-        for (int k = 0; k < 9; k++) m[k] = m[k] + C[k];
-    }
+    for (int k = SUM0 ? 1 : 0; k < 9; k++) m[k] = m[k] - P.Lf[k] * (m[k] - meq[k]) + P.relax_f[k] * S[k];
+    term(m);
     mul_Mi<D2Q9T>(P, m, f);
 }
 MPLB_HD void collide_limrt(const Params& P, double* f, double rho, const double* U, const double* F,
@@ -414,8 +428,9 @@ MPLB_HD void collide_limrt(const Params& P, double* f, double rho, const double*
 
 // xuMRTCollision.c:46-89, xuMRTEquilibriumMS.c:12-51, xuMRTForce.c:14-69.
 // F here is Fi + (rho - rho_0) g (no fext), xuMRTForce.c:18-22.
+template <bool SUM0 = false, class Term = NoTerm>
 MPLB_HD void collide_xumrt_psi(const Params& P, double* f, double rho, const double* U,
-                               const double* Fi, double ps, const double* C = nullptr) {
+                               const double* Fi, double ps, Term term = Term()) {
     double um = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) um += U[k] * U[k];
@@ -435,9 +450,10 @@ MPLB_HD void collide_xumrt_psi(const Params& P, double* f, double rho, const dou
     meq[12] = rho * U[1] * U[2];
     meq[13] = rho * U[0] * U[2];
     meq[14] = 0;
-    mul_M<D3Q15T>(f, m);
+    mul_M<D3Q15T, SUM0 ? 1 : 0>(f, m);
+    if (SUM0) m[0] = rho;
 #pragma unroll
-    for (int j = 0; j < 3; j++) F[j] = Fi[j] + (rho - P.rho_0) * P.g[j];
+    for (int j = 0; j < 3; j++) F[j] = SUM0 && !P.body ? Fi[j] : Fi[j] + (rho - P.rho_0) * P.g[j];
     double uf = U[0] * F[0] + U[1] * F[1] + U[2] * F[2];
     double f2 = 0;
 #pragma unroll
@@ -458,11 +474,8 @@ MPLB_HD void collide_xumrt_psi(const Params& P, double* f, double rho, const dou
     S[13] = U[0] * F[2] + U[2] * F[0];
     S[14] = 0;
 #pragma unroll
-    for (int k = 0; k < 15; k++) m[k] = m[k] - P.Lf[k] * (m[k] - meq[k]) + P.relax_f[k] * S[k];
-    if (C) {
-#pragma unroll
-        for (int k = 0; k < 15; k++) m[k] = m[k] + C[k];
-    }
+    for (int k = SUM0 ? 1 : 0; k < 15; k++) m[k] = m[k] - P.Lf[k] * (m[k] - meq[k]) + P.relax_f[k] * S[k];
+    term(m);
     mul_Mi<D3Q15T>(P, m, f);
 }
 MPLB_HD void collide_xumrt(const Params& P, double* f, double rho, const double* U, const double* Fi, double T) {
@@ -470,6 +483,8 @@ MPLB_HD void collide_xumrt(const Params& P, double* f, double rho, const double*
 }
 
 // liTempMRTCollision.c:38-84, liTempMRTEquilibriumMS.c:20-38, liTempMRTSource.c:17-24.
+// SUM0: T is the sum of g in k order (the fused steps).
+template <bool SUM0 = false>
 MPLB_HD void collide_litemp(const Params& P, double* g, double T, double u0, double u1, double src) {
     double neq[9], n[9];
     neq[0] = T;
@@ -481,9 +496,9 @@ MPLB_HD void collide_litemp(const Params& P, double* g, double T, double u0, dou
     neq[6] = T * (-u1);
     neq[7] = 0;
     neq[8] = 0;
-    mul_M<D2Q9T>(g, n);
+    mul_M<D2Q9T, SUM0 ? 1 : 0>(g, n);
     double n4 = n[4], n6 = n[6];
-    n[0] = n[0] - P.Lg[0] * (n[0] - neq[0]) + src;
+    n[0] = SUM0 ? T + src : n[0] - P.Lg[0] * (n[0] - neq[0]) + src;
 #pragma unroll
     for (int k = 1; k < 9; k++) n[k] = n[k] - P.Lg[k] * (n[k] - neq[k]) + 0.0;
     n[3] = n[3] + P.corr3 * n4;
@@ -563,16 +578,22 @@ MPLB_HD double heat_source_value(const Params& P, double rho, double T, double d
     double s = -lambda * dot / P.Cv + divU * T * (1.0 - dpdT / (rho * P.Cv));
     return s + 0.5 * (s - oldss);
 }
-// Same value, with the density's EOS parts er and rr = RN(1/rho) shared.
-MPLB_HD double heat_source_value_er(const Params& P, const EosRho& er, double rho, double rr, double T,
-                                    double dot, double divU, double oldss) {
-    double lambda = rho * P.Cv * P.lam_fac;
+// Same value in two parts, with the density's EOS parts er and rr = RN(1/rho)
+// shared: the one that needs no neighbour, and the rest.
+MPLB_HD double heat_eos_part(const Params& P, const EosRho& er, double rho, double rr, double T) {
     double dpdT = p_eos_at(P, er, rho, 1.1 * T) - p_eos_at(P, er, rho, 0.9 * T);
     dpdT = dpdT / (0.2 * T);
+    return P.cv_one ? div_rcp(dpdT, rho, rr) : dpdT / (rho * P.Cv);
+}
+MPLB_HD double heat_source_from(const Params& P, double rho, double T, double dot, double divU, double b, double oldss) {
+    double lambda = rho * P.Cv * P.lam_fac;
     double a = P.cv_one ? -lambda * dot : -lambda * dot / P.Cv;
-    double b = P.cv_one ? div_rcp(dpdT, rho, rr) : dpdT / (rho * P.Cv);
     double s = a + divU * T * (1.0 - b);
     return s + 0.5 * (s - oldss);
+}
+MPLB_HD double heat_source_value_er(const Params& P, const EosRho& er, double rho, double rr, double T,
+                                    double dot, double divU, double oldss) {
+    return heat_source_from(P, rho, T, dot, divU, heat_eos_part(P, er, rho, rr, T), oldss);
 }
 
 // ------------------------------------------------------- dependent launch

@@ -1049,6 +1049,10 @@ int mplb_gpu_create(const mplb_mesh_desc* mesh, const mplb_eos_desc* eos, const 
     P.Cv = eos->Cv;
     P.rho_0 = eos->rho_0;
     for (int j = 0; j < 3; j++) { P.g[j] = eos->g[j]; P.fext[j] = eos->fext[j]; }
+    P.body = P.body_z = 0;
+    for (int j = 0; j < 3; j++)
+        if (eos->g[j] != 0.0 || eos->fext[j] != 0.0) P.body = 1;
+    if (eos->g[2] != 0.0 || eos->fext[2] != 0.0) P.body_z = 1;
     P.g_neg1 = eos->G == -1.0;
     P.cv_one = eos->Cv == 1.0;
     P.m2_one = eos->M * eos->M == 1.0;

@@ -64,29 +64,26 @@ __global__ void k_collide_flow(Params P, double* __restrict__ f, const double* _
     const double ps = potential(P, rho[id], T[id]);
     // surface-tension term: zero on a node with any missing neighbour
     // (liMRTSurfaceTension.c:33-45), else from psi at x + c_k = nb[rev k]
-    double C[L::Q];
-    const double* Cp = nullptr;
-    if (P.st_on) {
+    auto term = [&](double* m) {
+        if (!P.st_on) return;
         bool interior = true;
 #pragma unroll
         for (int k = 1; k < L::Q; k++) interior &= nb[(size_t)k * n + id] != -1;
-        if (interior) {
-            auto nbpsi = [&](int k) {
-                const uint32_t m = (uint32_t)nb[(size_t)revk<L>(k) * n + id];
-                return potential(P, rho[m], T[m]);
-            };
-            surface_tension<L>(P, ps, nbpsi, C);
-        } else {
+        if (!interior) return;
+        auto nbpsi = [&](int k) {
+            const uint32_t q = (uint32_t)nb[(size_t)revk<L>(k) * n + id];
+            return potential(P, rho[q], T[q]);
+        };
+        double C[L::Q];
+        surface_tension<L>(P, ps, nbpsi, C);
 #pragma unroll
-            for (int k = 0; k < L::Q; k++) C[k] = 0;
-        }
-        Cp = C;
-    }
+        for (int k = 0; k < L::Q; k++) m[k] = m[k] + C[k];
+    };
     if constexpr (L::Q == 9) {
         double ft[3] = {Ft[id], Ft[n + id], Ft[2 * n + id]};
-        collide_limrt_psi(P, v, rho[id], u, ft, fi, ps, Cp);
+        collide_limrt_psi(P, v, rho[id], u, ft, fi, ps, term);
     } else {
-        collide_xumrt_psi(P, v, rho[id], u, fi, ps, Cp);
+        collide_xumrt_psi(P, v, rho[id], u, fi, ps, term);
     }
 #pragma unroll
     for (int k = 0; k < L::Q; k++) f[(size_t)k * n + id] = v[k];
