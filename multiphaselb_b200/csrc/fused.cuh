@@ -73,6 +73,8 @@ struct FusedArgs {
     double* Ft_out;
     const uint8_t* bcmap;  // per node: 0 = no boundary op, else index into prog
     int bc_margin;         // largest distance of a node with a boundary op from its nearest face, -1 = none
+    int mx, my;            // 2D: every wall node and every node with a boundary op lies within mx of an x face
+                           // or within my of a y face (-1: none does)
     int* kerr;             // kernel-side error flag (a bounded wait that ran out), read by the host
     double* rho_a;         // myMRT thermal field: rho_n and sum g''_n of every node (k_pullsum_d2q9)
     double* gsum_a;
@@ -82,6 +84,14 @@ struct FusedArgs {
     double Twall[MPLB_MAX_PATCHES];
     BCProg prog[FUSED_MAX_PROGS];
 };
+
+__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
 // ------------------------------------------------------------- geometry
 // Wrap a coordinate one step outside [0, ext): periodic -> wrapped,
@@ -514,7 +524,7 @@ __device__ __forceinline__ double heat_my(const Params& P, const FusedArgs& A, i
     double dot = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) dot += gT[k] * gR[k];
-    return heat_source_value_my(P, ri, Ti, dot, div);
+    return heat_source_value_my_er(P, eos_rho(P, ri), ri, rcp_rn(ri), Ti, dot, div);
 }
 
 // myMRT steps: rho_n and sum g''_n of every node (pull, boundary program,
@@ -813,13 +823,6 @@ __global__ void __launch_bounds__(F3_TX * F3_TY, min_blocks(F3_TX * F3_TY)) k_fu
 // never written.
 constexpr int F3_STAGES = 3;
 
-__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-
 template <int F3_TX, int F3_TY, bool HAS_BC, bool EMIT>
 __global__ void __launch_bounds__(F3_TX * F3_TY, min_blocks(F3_TX * F3_TY)) k_fused_d3q15_pipe(Params P, FusedArgs A) {
     step_dependency_wait();
@@ -954,12 +957,14 @@ struct TileCfg {
                  // on large lattices; a lattice of one wave prefers the smaller general kernel)
     bool tma;    // 3D only: planes staged by TMA (k_fused_d3q15_tma; fully periodic boxes)
     int ringw;   // 2D only: added warps that compute the ring (k_fused_d2q9 RINGW)
+    bool march;  // 2D myMRT heat only: the marching kernel (k_march_my_d2q9)
 };
-constexpr int N_CFG2 = 10, N_CFG3 = 10, N_CFG_MAX = 10;
+constexpr int N_CFG2 = 11, N_CFG3 = 10, N_CFG_MAX = 11;
 constexpr TileCfg CFG2[N_CFG2] = {{32, 8, false, 0, false}, {32, 4, false, 0, false}, {64, 4, false, 0, false},
                                   {16, 8, false, 0, true},  {64, 4, false, 0, true},  {16, 8, false, 6, true},
                                   {32, 8, false, 3, true},  {32, 4, false, 8, true},
-                                  {32, 8, false, 2, false, false, 3}, {16, 8, false, 4, false, false, 2}};
+                                  {32, 8, false, 2, false, false, 3}, {16, 8, false, 4, false, false, 2},
+                                  {28, 1, false, 0, false, false, 0, true}};
 constexpr TileCfg CFG3[N_CFG3] = {{32, 8, false, 0, false}, {32, 8, true, 0, false}, {32, 4, false, 0, false},
                                   {64, 4, false, 0, false}, {32, 16, false, 0, false}, {64, 8, false, 0, false},
                                   {32, 4, false, 3, false, true}, {32, 8, false, 2, false, true},

@@ -7,7 +7,12 @@
 #include <cudaTypedefs.h>
 
 #include "fused.cuh"
+#include "fused_march.cuh"
 #include "fused_tma.cuh"
+
+// The marching D2Q9 step with myMRT heat (mplb_march.cu).
+int mplb_march_resident(bool f_on, bool bc);
+cudaError_t mplb_march_launch(bool f_on, bool bc, int nb, const mplb::Params& P, const mplb::FusedArgs& A, cudaStream_t s);
 
 namespace mplb {
 
@@ -200,6 +205,8 @@ inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, F
             launch2_fg<32, 8, true>(f_on, g_on, bc, nb, P, A, s);
         } else if (st) {
             launch2_fg<32, 8, false, 0, false, 0, true>(f_on, g_on, bc, nb, P, A, s);
+        } else if (CFG2[cfg].march) {
+            return mplb_march_launch(f_on, bc, nb, P, A, s);
         } else {
             switch (cfg) {
             case 0: launch2_fg<32, 8, false>(f_on, g_on, bc, nb, P, A, s); break;
@@ -418,6 +425,18 @@ inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params&
         if (lat == MPLB_D3Q15) d = std::min(d, std::min(z, A.nz - 1 - z));
         A.bc_margin = std::max(A.bc_margin, d);
     }
+    // 2D: margins from the x and the y faces that together hold every wall node
+    // and every node with a program
+    A.mx = A.px ? -1 : 0;
+    A.my = A.py ? -1 : 0;
+    for (uint32_t id = 0; lat == MPLB_D2Q9 && id < n; id++) {
+        if (!map[id]) continue;
+        const int x = (int)(id % (uint32_t)A.nx), y = (int)(id / (uint32_t)A.nx);
+        const int dx = std::min(x, A.nx - 1 - x), dy = std::min(y, A.ny - 1 - y);
+        if (dx <= A.mx || dy <= A.my) continue;
+        if (dx < dy) A.mx = dx;
+        else A.my = dy;
+    }
     for (size_t q = 0; q < progs.size(); q++) A.prog[q] = progs[q];
     for (size_t p = 0; p < fp[1].size() && p < MPLB_MAX_PATCHES; p++) A.Twall[p] = fp[1][p].val[0];
     fc.has_bc = any;
@@ -447,6 +466,9 @@ inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params&
         const TileCfg t = lat == MPLB_D2Q9 ? CFG2[c] : CFG3[c];
         if (t.tma) {
             fc.geom[c] = tma3_fits(A, any, t.tx, t.ty) ? resident_geometry(A, t.tx, t.ty, t.minb) : Geom{0, 0, 0, 0};
+        } else if (t.march) {
+            const bool my = P.g_update && model[1] == MPLB_MYMRT;
+            fc.geom[c] = my ? march_geometry(A, mplb_march_resident(P.f_update != 0, any)) : Geom{0, 0, 0, 0};
         } else {
             fc.geom[c] = fused_geometry(lat, A, t.tx, t.ty);
         }

@@ -95,6 +95,7 @@ struct Params {
     double my_qo[3];             // off-diagonal rates Q[3][4], Q[5][6], Q[7][8]   myMRTCollision.c:80-116
     double my_qa0;               // (I - Q/2)[0][0] = 1.0 + (-0.5*Lambda[0])      myMRTCollision.c:125-140
     double my_lgeo, my_ldiv;     // conductivity factor: (4 + 3a1 + 2a2), 6 (D2Q9); (6 + 11a1 + a2), 9 (D3Q15)
+    double my_ldivr;             // RN(1/my_ldiv)
     // EOS (EOSInfo.h:80-102)
     int32_t eos;
     double a, b, R, G, M, Cv, rho_0;
@@ -567,6 +568,19 @@ MPLB_HD double heat_source_value_my(const Params& P, double rho, double T, doubl
     double dpdT = p_eos(P, rho, 1.1 * T) - p_eos(P, rho, 0.9 * T);
     dpdT = dpdT / (0.2 * T);
     return -lambda * dot / P.Cv + divU * T * (1.0 - dpdT / (rho * P.Cv));
+}
+
+// Same value with the density's EOS parts er and rr = RN(1/rho) shared, and
+// the division by the constant 6 or 9 through its reciprocal (div_rcp): one
+// full division instead of five or six.
+MPLB_HD double heat_source_value_my_er(const Params& P, const EosRho& er, double rho, double rr, double T, double dot,
+                                       double divU) {
+    double lambda = div_rcp(rho * P.Cv * P.lam_fac * P.my_lgeo, P.my_ldiv, P.my_ldivr);
+    double dpdT = p_eos_at(P, er, rho, 1.1 * T) - p_eos_at(P, er, rho, 0.9 * T);
+    dpdT = dpdT / (0.2 * T);
+    double a = P.cv_one ? -lambda * dot : -lambda * dot / P.Cv;
+    double b = P.cv_one ? div_rcp(dpdT, rho, rr) : dpdT / (rho * P.Cv);
+    return a + divU * T * (1.0 - b);
 }
 
 // heatSource.c:144-165: source from gradients (dot), divergence, rho, T_old.

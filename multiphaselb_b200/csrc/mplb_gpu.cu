@@ -1038,6 +1038,7 @@ int mplb_gpu_create(const mplb_mesh_desc* mesh, const mplb_eos_desc* eos, const 
                 P.my_lgeo = 6.0 + 11.0 * g->alpha_1 + g->alpha_2;
                 P.my_ldiv = 9.0;
             }
+            P.my_ldivr = 1.0 / P.my_ldiv;
         }
     }
     P.eos = eos->type;
