@@ -296,11 +296,26 @@ __device__ __forceinline__ void pull_node(const Params& P, const FusedArgs& A, i
 }
 
 // ------------------------------------------------------------ phase B
+// sum_k c_k f_k, the terms of zero velocity components skipped (they are +-0).
+template <class L>
+__device__ __forceinline__ void momentum(const double* f, double* lv) {
+    static_for<L::D>([&](auto jj) {
+        constexpr int j = decltype(jj)::value;
+        double v = 0;
+        static_for<L::Q>([&](auto kk) {
+            constexpr int c = ck<L>(decltype(kk)::value, j);
+            if constexpr (c == 1) v = v + f[kk];
+            else if constexpr (c == -1) v = v - f[kk];
+        });
+        lv[j] = v;
+    });
+}
+
 // Interaction force, total force and velocity of one node from its
-// post-stream populations f, density rho (rr = RN(1/rho)) and psi
-// (nbpsi(k) = psi_n at x + c_k).
+// momentum lv (sum_k c_k f_k; D components), density rho (rr = RN(1/rho)) and
+// psi (nbpsi(k) = psi_n at x + c_k).
 template <class L, bool EMIT, class PsiAt>
-__device__ __forceinline__ void force_velocity(const Params& P, bool onb, const double* f, double rho, double rr,
+__device__ __forceinline__ void force_velocity(const Params& P, bool onb, const double* lv, double rho, double rr,
                                                double psi, PsiAt nbpsi, double* Fi, double* Ft, double* U) {
     Fi[0] = Fi[1] = Fi[2] = 0;
     // interactionForce.c:47-79 (zero force on boundary nodes)
@@ -333,7 +348,6 @@ __device__ __forceinline__ void force_velocity(const Params& P, bool onb, const 
         for (int j = 0; j < 3; j++) Ft[j] = Fi[j];
     }
     // liMRTVelocity.c:27-44 (F = Ft) / xuMRTVelocity.c:19-44 (F = Fi + (rho - rho_0) g).
-    // Zero velocity components contribute +-0 and are skipped.
     // In 2D the third component is zero unless a body force acts along it.
     static_for<3>([&](auto jj) {
         constexpr int j = decltype(jj)::value;
@@ -341,14 +355,8 @@ __device__ __forceinline__ void force_velocity(const Params& P, bool onb, const 
             U[j] = 0;
             return;
         }
-        double lv = 0;
-        static_for<L::Q>([&](auto kk) {
-            constexpr int c = ck<L>(decltype(kk)::value, j);
-            if constexpr (c == 1) lv = lv + f[kk];
-            else if constexpr (c == -1) lv = lv - f[kk];
-        });
         double Fj = L::Q == 9 ? Ft[j] : (EMIT || P.body ? Fi[j] + (rho - P.rho_0) * P.g[j] : Fi[j]);
-        U[j] = div_rcp(lv + Fj * 0.5, rho, rr);  // == (lv + Fj*0.5)/rho
+        U[j] = div_rcp((j < L::D ? lv[j < L::D ? j : 0] : 0.0) + Fj * 0.5, rho, rr);  // == (lv + Fj*0.5)/rho
     });
 }
 
@@ -371,7 +379,9 @@ __device__ __forceinline__ void finish_node(const Params& P, const FusedArgs& A,
         if (id - A.own_lo >= A.own_cnt) return;
     double Fi[3] = {0, 0, 0}, Ft[3], U[3];
     if constexpr (F_ON) {
-        force_velocity<L, EMIT>(P, onb, f, rho, rr, psi, nbpsi, Fi, Ft, U);
+        double lv[L::D];
+        momentum<L>(f, lv);
+        force_velocity<L, EMIT>(P, onb, lv, rho, rr, psi, nbpsi, Fi, Ft, U);
     } else {
 #pragma unroll
         for (int j = 0; j < 3; j++) U[j] = A.Uold[(size_t)j * n + id];

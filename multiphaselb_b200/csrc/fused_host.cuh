@@ -59,39 +59,40 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// The maps of TMA candidate `cfg` for the step's input buffers: the
-// populations as a 4D tensor (x, y, z, k) and T as a 3D one (x, y, z), FP64,
-// boxes of (TX+4) x (TY+2) x 1 (x 1), no swizzle, zero fill (never read: the
-// kernel takes tensor copies only for boxes inside the lattice).
-inline const TmaMaps* tma_maps(FusedConfig& fc, int cfg, const FusedArgs& A, uint32_t n) {
+// Tensor maps of a step's input buffers: the populations (FP64 or FP32) as a
+// 4D tensor (x, y, z, k) with boxes of bx x by, T as a 3D one (x, y, z) with
+// boxes of tbx x by; no swizzle, zero fill (never read: the kernels take
+// tensor copies only for boxes inside the lattice).  Kept per (key, buffers).
+inline const TmaMaps* tma_maps(FusedConfig& fc, int key, const FusedArgs& A, const void* fin, bool fp32,
+                               const double* Told, uint32_t n, int bx, int by, int tbx) {
     for (const TmaMaps& m : fc.tmaps)
-        if (m.cfg == cfg && m.f == A.fin && m.T == A.Told) return &m;
+        if (m.cfg == key && m.f == fin && m.T == Told) return &m;
     auto enc = tensor_map_encoder();
     if (!enc) {
         fc.err = "cuTensorMapEncodeTiled is not available from the driver";
         return nullptr;
     }
     TmaMaps& m = fc.tmaps[fc.tmaps_next];
-    const TileCfg t = CFG3[cfg];
     const cuuint64_t dims[4] = {(cuuint64_t)A.nx, (cuuint64_t)A.ny, (cuuint64_t)A.nz, 15};
-    const cuuint64_t strides[3] = {(cuuint64_t)A.nx * 8, (cuuint64_t)A.nx * A.ny * 8, (cuuint64_t)n * 8};
-    const cuuint32_t box[4] = {(cuuint32_t)(t.tx + 4), (cuuint32_t)(t.ty + 2), 1, 1};
-    const cuuint32_t es[4] = {1, 1, 1, 1};
-    CUresult r = enc(&m.mf, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<double*>(A.fin), dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r == CUDA_SUCCESS)
-        r = enc(&m.mT, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double*>(A.Told), dims, strides, box, es,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto encode = [&](CUtensorMap* map, bool f32, int rank, const void* p, int width) {
+        const cuuint64_t es = f32 ? 4 : 8;
+        const cuuint64_t strides[3] = {(cuuint64_t)A.nx * es, (cuuint64_t)A.nx * A.ny * es, (cuuint64_t)n * es};
+        const cuuint32_t box[4] = {(cuuint32_t)width, (cuuint32_t)by, 1, 1};
+        const cuuint32_t step[4] = {1, 1, 1, 1};
+        return enc(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, rank,
+                   const_cast<void*>(p), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode(&m.mf, fp32, 4, fin, bx);
+    if (r == CUDA_SUCCESS) r = encode(&m.mT, false, 3, Told, tbx);
     if (r != CUDA_SUCCESS) {
         fc.err = "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")";
         m.cfg = -1;
         return nullptr;
     }
-    m.cfg = cfg;
-    m.f = A.fin;
-    m.T = A.Told;
+    m.cfg = key;
+    m.f = fin;
+    m.T = Told;
     fc.tmaps_next = (fc.tmaps_next + 1) % 4;
     return &m;
 }
@@ -137,7 +138,7 @@ inline cudaError_t fused_attributes() {
 
 template <int TX, int TY, int MINB>
 cudaError_t launch3_tma(FusedConfig& fc, int cfg, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
-    const TmaMaps* m = tma_maps(fc, cfg, A, P.n);
+    const TmaMaps* m = tma_maps(fc, cfg, A, A.fin, false, A.Told, P.n, TX + 4, TY + 2, TX + 4);
     if (!m) return cudaErrorInvalidValue;
     if (P.st_on) launch_step(k_fused_d3q15_tma<TX, TY, MINB, true>, nb, TX * TY, TmaTile<TX, TY>::SMEM, s, P, A, m->mf, m->mT);
     else launch_step(k_fused_d3q15_tma<TX, TY, MINB>, nb, TX * TY, TmaTile<TX, TY>::SMEM, s, P, A, m->mf, m->mT);

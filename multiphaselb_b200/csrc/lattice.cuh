@@ -429,13 +429,15 @@ MPLB_HD void collide_limrt(const Params& P, double* f, double rho, const double*
 
 // xuMRTCollision.c:46-89, xuMRTEquilibriumMS.c:12-51, xuMRTForce.c:14-69.
 // F here is Fi + (rho - rho_0) g (no fext), xuMRTForce.c:18-22.
+// relax_xumrt: the part after m = M f (with SUM0, moments 1 to 14); f is
+// written only.
 template <bool SUM0 = false, class Term = NoTerm>
-MPLB_HD void collide_xumrt_psi(const Params& P, double* f, double rho, const double* U,
-                               const double* Fi, double ps, Term term = Term()) {
+MPLB_HD void relax_xumrt(const Params& P, double* m, double* f, double rho, const double* U, const double* Fi,
+                         double ps, Term term = Term()) {
     double um = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) um += U[k] * U[k];
-    double meq[15], m[15], S[15], F[3];
+    double meq[15], S[15], F[3];
     meq[0] = rho;
     meq[1] = rho * (-1.0 + um);
     meq[2] = rho * (1.0 - 5.0 * um);
@@ -451,7 +453,6 @@ MPLB_HD void collide_xumrt_psi(const Params& P, double* f, double rho, const dou
     meq[12] = rho * U[1] * U[2];
     meq[13] = rho * U[0] * U[2];
     meq[14] = 0;
-    mul_M<D3Q15T, SUM0 ? 1 : 0>(f, m);
     if (SUM0) m[0] = rho;
 #pragma unroll
     for (int j = 0; j < 3; j++) F[j] = SUM0 && !P.body ? Fi[j] : Fi[j] + (rho - P.rho_0) * P.g[j];
@@ -478,6 +479,13 @@ MPLB_HD void collide_xumrt_psi(const Params& P, double* f, double rho, const dou
     for (int k = SUM0 ? 1 : 0; k < 15; k++) m[k] = m[k] - P.Lf[k] * (m[k] - meq[k]) + P.relax_f[k] * S[k];
     term(m);
     mul_Mi<D3Q15T>(P, m, f);
+}
+template <bool SUM0 = false, class Term = NoTerm>
+MPLB_HD void collide_xumrt_psi(const Params& P, double* f, double rho, const double* U, const double* Fi, double ps,
+                               Term term = Term()) {
+    double m[15];
+    mul_M<D3Q15T, SUM0 ? 1 : 0>(f, m);
+    relax_xumrt<SUM0>(P, m, f, rho, U, Fi, ps, term);
 }
 MPLB_HD void collide_xumrt(const Params& P, double* f, double rho, const double* U, const double* Fi, double T) {
     collide_xumrt_psi(P, f, rho, U, Fi, potential(P, rho, T));

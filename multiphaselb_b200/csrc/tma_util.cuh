@@ -32,6 +32,18 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// add to the bytes this phase waits for, without arriving
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// arrive once every cp.async this thread has issued so far has landed
+__device__ __forceinline__ void mbar_arrive_cp_async(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// 16 bytes from global to shared memory, both 16-byte aligned
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 // true once the phase with this parity has completed
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
@@ -71,7 +83,56 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  : "memory");
 }
 
+// order this thread's earlier shared-memory accesses before later async-proxy (TMA) writes
+__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // c within one extent of [0, ext): wrapped into it
 MPLB_HD int wrap_any(int c, int ext) { return c < 0 ? c + ext : (c >= ext ? c - ext : c); }
+
+// Wrapped parts of a plane stage.  A stage holds NBOX boxes of BY rows; box b
+// starts at row y0 - 1 - cy_b, and every row reaches 16 bytes past the tile's
+// TX columns on either side (two doubles, four floats), so in bytes all boxes
+// are alike.  A tensor copy fills the parts outside the lattice with zeros;
+// this writes the periodic images there: for tiles on an x face the 16 bytes
+// of every row (one thread each), for tiles on a y face the one or two rows of
+// a box that lie outside (one thread and one bulk copy each).  The work goes to
+// the block's last warps; its first ones have the ring.  row(b, iy, y, dst,
+// src, es) gives row iy of box b in shared memory, the start of lattice row y of
+// its plane, and the element size; cy(b) is the box's shift; copy(dst, src)
+// copies 16 bytes, bulk(dst, src, bytes) a multiple of 16.
+template <int TX, int TY, int NBOX, class Cy, class Row, class Copy, class Bulk>
+MPLB_HD void patch_wrapped(int tid, int nt, int x0, int y0, int nx, int ny, Cy cy, Row row, Copy copy, Bulk bulk) {
+    constexpr int BY = TY + 2, NROWS = NBOX * BY;
+    const bool left = x0 == 0, right = x0 + TX == nx;
+    unsigned char* dst;
+    const unsigned char* src;
+    int es;
+    const int t = nt - 1 - tid;
+    if (left || right) {
+        for (int r = t; r < NROWS; r += nt) {
+            const int b = r / BY, iy = r - b * BY, y = y0 - 1 - cy(b) + iy;
+            if (y < 0 || y >= ny) continue;  // a row of the second part
+            row(b, iy, y, dst, src, es);
+            if (left) copy(dst, src + nx * es - 16);
+            if (right) copy(dst + 16 + TX * es, src);
+        }
+    }
+    // rows outside: per box and side, at most two; the warp below the x part's
+    const int yt = t - (NROWS + 31 < nt ? (NROWS + 31) / 32 * 32 : nt - 32);
+    static_assert(2 * NBOX <= 32, "one lane per row");
+    if (yt < 0 || yt >= 2 * NBOX) return;
+    for (int side = 0; side < 2; side++) {
+        if (side ? y0 + TY != ny : y0 != 0) continue;
+        const int b = yt >> 1, w = yt & 1;
+        if (w >= (side ? 1 - cy(b) : 1 + cy(b))) continue;
+        const int iy = side ? BY - 1 - w : w;
+        row(b, iy, wrap_any(y0 - 1 - cy(b) + iy, ny), dst, src, es);
+        const int lo = left ? 16 : 0, hi = 32 + TX * es - (right ? 16 : 0);  // the part inside the box in x
+        bulk(dst + lo, src + (x0 * es - 16 + lo), hi - lo);
+        if (left) copy(dst, src + nx * es - 16);
+        if (right) copy(dst + 16 + TX * es, src);
+    }
+}
 
 }  // namespace mplb
