@@ -38,18 +38,21 @@ struct FusedArgs32 {
     // FP32 copies of the collision constants
     float Lf[MPLB_MAX_Q], relax_f[MPLB_MAX_Q], Lg[9];
     float s1_den, s2_den, sig12, sig6, corr3, corr5;
+    int* kerr;      // FusedArgs::kerr
     const uint8_t* bcmap;
     int bc_margin;  // FusedArgs::bc_margin
     double Twall[MPLB_MAX_PATCHES];
     BCProg prog[FUSED_MAX_PROGS];
 };
 
-template <class L>
+// FIRST: the first row to evaluate (row 0, the sum, may be known already).
+template <class L, int FIRST = 0>
 __device__ __forceinline__ void mul_M32(const float* v, float* r) {
-    static_for<L::Q>([&](auto i) {
+    static_for<L::Q - FIRST>([&](auto im) {
+        constexpr int i = decltype(im)::value + FIRST;
         float s = 0.f;
         static_for<L::Q>([&](auto j) {
-            constexpr int c = Mint<L>(decltype(i)::value, decltype(j)::value);
+            constexpr int c = Mint<L>(i, decltype(j)::value);
             if constexpr (c == 1) s += v[j];
             else if constexpr (c == -1) s -= v[j];
             else if constexpr (c != 0) s += (float)c * v[j];
@@ -111,25 +114,46 @@ constexpr int axis_population(int d) {
     return 0;
 }
 
+// Mass and momentum of FP32 populations in FP64: rest = mass without the axis
+// populations, axis = mass of the axis ones, mom = momentum.  The sums of
+// opposite signs share their partial sums (FP64 sums of FP32 values are exact,
+// so the grouping does not matter); each population is converted once.
+template <class L>
+__device__ __forceinline__ void exact_moments(const float* f, double& rest, double& axis, double* mom) {
+    double d[L::Q];
+#pragma unroll
+    for (int k = 0; k < L::Q; k++) d[k] = (double)f[k];
+    if constexpr (L::Q == 9) {
+        const double a = d[5] + d[6], b = d[7] + d[8];
+        rest = d[0] + (a + b);
+        axis = (d[1] + d[3]) + (d[2] + d[4]);
+        mom[0] = (d[1] - d[3]) + ((d[5] - d[6]) + (d[8] - d[7]));
+        mom[1] = (d[2] - d[4]) + (a - b);
+    } else {
+        const double s1 = d[7] + d[8], s2 = d[9] + d[10], s3 = d[11] + d[12], s4 = d[13] + d[14];
+        const double zp = s1 + s2, zm = s3 + s4;
+        rest = d[0] + (zp + zm);
+        axis = ((d[1] + d[2]) + (d[3] + d[4])) + (d[5] + d[6]);
+        mom[0] = (d[1] - d[2]) + (((d[7] - d[8]) + (d[9] - d[10])) + ((d[11] - d[12]) + (d[13] - d[14])));
+        mom[1] = (d[3] - d[4]) + ((s1 - s2) + (s3 - s4));
+        mom[2] = (d[5] - d[6]) + (zp - zm);
+    }
+}
+
 template <class L>
 __device__ __forceinline__ void restore_conserved(float* f, double mass, const double* mom) {
+    double rest, axis, j[3];
+    exact_moments<L>(f, rest, axis, j);
+    axis = 0.0;
     static_for<L::D>([&](auto dd) {
         constexpr int d = decltype(dd)::value;
-        double j = 0.0;
-        static_for<L::Q>([&](auto kk) {
-            constexpr int c = ck<L>(decltype(kk)::value, d);
-            if constexpr (c == 1) j += (double)f[kk];
-            else if constexpr (c == -1) j -= (double)f[kk];
-        });
-        const double half = 0.5 * (mom[d] - j);
+        const double half = 0.5 * (mom[d] - j[d]);
         constexpr int a = axis_population<L>(d), b = revk<L>(a);
         f[a] = (float)((double)f[a] + half);
         f[b] = (float)((double)f[b] - half);
+        axis += (double)f[a] + (double)f[b];
     });
-    double post = 0.0;
-#pragma unroll
-    for (int k = 0; k < L::Q; k++) post += (double)f[k];
-    const double v = (double)f[0] + (mass - post);
+    const double v = (double)f[0] + (mass - (rest + axis));
     f[0] = (float)v;
     const double half = 0.5 * (v - (double)f[0]);
     constexpr int a = first_diagonal<L>(), b = revk<L>(a);
@@ -208,13 +232,14 @@ __device__ __forceinline__ void momentum_fix_node(float* __restrict__ f, uint32_
     });
 }
 
-// liMRT collision on deviations (liMRTCollision.c / liMRTForce.c in FP32).
-__device__ __forceinline__ void collide_limrt32(const FusedArgs32& A, float* f, double rho, float dr, const float* U,
-                                                const float* F, const float* Fi, double psi) {
+// liMRT collision on deviations (liMRTCollision.c / liMRTForce.c in FP32); m
+// holds the moments, f is written only.  Moment 0 is dr, equal to its
+// equilibrium, and has no source.
+__device__ __forceinline__ void collide_limrt32(const FusedArgs32& A, float* m, float* f, double rho, float dr,
+                                                const float* U, const float* F, const float* Fi, double psi) {
     const float r = (float)rho;
     const float um = U[0] * U[0] + U[1] * U[1] + U[2] * U[2];
-    float meq[9], m[9], S[9];
-    meq[0] = dr;
+    float meq[9], S[9];
     meq[1] = -2.f * dr + 3.f * r * um;
     meq[2] = dr - 3.f * r * um;
     meq[3] = r * U[0];
@@ -223,11 +248,9 @@ __device__ __forceinline__ void collide_limrt32(const FusedArgs32& A, float* f, 
     meq[6] = -r * U[1];
     meq[7] = r * (U[0] * U[0] - U[1] * U[1]);
     meq[8] = r * U[0] * U[1];
-    mul_M32<D2Q9T>(f, m);
     const float ps2 = (float)(psi * psi);
     const float uf = U[0] * F[0] + U[1] * F[1];
     const float fi2 = Fi[0] * Fi[0] + Fi[1] * Fi[1];
-    S[0] = 0.f;
     S[1] = 6.f * uf + A.sig12 * fi2 / (ps2 * A.s1_den);
     S[2] = -6.f * uf - A.sig12 * fi2 / (ps2 * A.s2_den);
     S[3] = F[0];
@@ -237,18 +260,18 @@ __device__ __forceinline__ void collide_limrt32(const FusedArgs32& A, float* f, 
     S[7] = 2.f * (U[0] * F[0] - U[1] * F[1]);
     S[8] = U[0] * F[1] + U[1] * F[0];
 #pragma unroll
-    for (int k = 0; k < 9; k++) m[k] = m[k] - A.Lf[k] * (m[k] - meq[k]) + A.relax_f[k] * S[k];
+    for (int k = 1; k < 9; k++) m[k] = m[k] - A.Lf[k] * (m[k] - meq[k]) + A.relax_f[k] * S[k];
+    m[0] = dr;
     mul_Mi32<D2Q9T>(m, f);
 }
 
 // xuMRT collision on deviations.
-__device__ __forceinline__ void collide_xumrt32(const FusedArgs32& A, float* f, double rho, float dr, const float* U,
-                                                const float* F, double psi) {
+__device__ __forceinline__ void collide_xumrt32(const FusedArgs32& A, float* m, float* f, double rho, float dr,
+                                                const float* U, const float* F, double psi) {
     const float r = (float)rho;
     const float um = U[0] * U[0] + U[1] * U[1] + U[2] * U[2];
     constexpr float S73 = 7.f / 3.f;
-    float meq[15], m[15], S[15];
-    meq[0] = dr;
+    float meq[15], S[15];
     meq[1] = -dr + r * um;
     meq[2] = dr - 5.f * r * um;
     meq[3] = r * U[0];
@@ -263,10 +286,8 @@ __device__ __forceinline__ void collide_xumrt32(const FusedArgs32& A, float* f, 
     meq[12] = r * U[1] * U[2];
     meq[13] = r * U[0] * U[2];
     meq[14] = 0.f;
-    mul_M32<D3Q15T>(f, m);
     const float uf = U[0] * F[0] + U[1] * F[1] + U[2] * F[2];
     const float f2 = F[0] * F[0] + F[1] * F[1] + F[2] * F[2];
-    S[0] = 0.f;
     S[1] = 2.f * uf + A.sig6 * f2 / ((float)(psi * psi) * A.s1_den);
     S[2] = -10.f * uf;
     S[3] = F[0];
@@ -282,7 +303,8 @@ __device__ __forceinline__ void collide_xumrt32(const FusedArgs32& A, float* f, 
     S[13] = U[0] * F[2] + U[2] * F[0];
     S[14] = 0.f;
 #pragma unroll
-    for (int k = 0; k < 15; k++) m[k] = m[k] - A.Lf[k] * (m[k] - meq[k]) + A.relax_f[k] * S[k];
+    for (int k = 1; k < 15; k++) m[k] = m[k] - A.Lf[k] * (m[k] - meq[k]) + A.relax_f[k] * S[k];
+    m[0] = dr;
     mul_Mi32<D3Q15T>(m, f);
 }
 
@@ -446,49 +468,118 @@ __device__ __forceinline__ void prefetch_node32(const FusedArgs32& A, int x, int
     }
 }
 
+// What a node's collision needs of its populations, before its neighbours'
+// psi: exact mass and momentum, and the FP32 moments 1 to Q-1 (3, 5, 7 are the
+// momentum summed in FP32, from which the velocity is taken).
+template <class L>
+struct Pre32 {
+    double mass, mom[3];
+    float m[L::Q];
+};
+template <class L>
+__device__ __forceinline__ void pre_node32(const float* f, Pre32<L>& q) {
+    double rest, axis;
+    exact_moments<L>(f, rest, axis, q.mom);
+    q.mass = rest + axis;
+    mul_M32<L, 1>(f, q.m);
+}
+
+// The rows of the momentum alone (3, 5, 7), as mul_M32 sums them.
+template <class L>
+__device__ __forceinline__ void momentum32(const float* f, float* m) {
+    static_for<L::D>([&](auto dd) {
+        constexpr int d = decltype(dd)::value;
+        float s = 0.f;
+        static_for<L::Q>([&](auto kk) {
+            constexpr int c = ck<L>(decltype(kk)::value, d);
+            if constexpr (c == 1) s += f[kk];
+            else if constexpr (c == -1) s -= f[kk];
+        });
+        m[3 + 2 * d] = s;
+    });
+}
+
+// Interaction force, total force and velocity in FP64 from the moments m
+// (sum_k c_k f_k of the deviations is that of the populations: sum_k c_k w_k = 0).
+template <class L, class PsiAt>
+__device__ __forceinline__ void force_velocity32(const Params& P, bool onb, const float* m, double rho, double psi,
+                                                 PsiAt nbpsi, double* Fi, double* Ft, double* Ud) {
+    Fi[0] = Fi[1] = Fi[2] = 0;
+    if (!onb) {
+        double F[3] = {0.0, 0.0, 0.0};
+        static_for<L::Q - 1>([&](auto km1) {
+            constexpr int k = decltype(km1)::value + 1;
+            const double al = P.ppw[k] * nbpsi(k);
+            static_for<3>([&](auto i) {
+                constexpr int c = ck<L>(k, decltype(i)::value);
+                if constexpr (c == 1) F[i] += al;
+                else if constexpr (c == -1) F[i] -= al;
+            });
+        });
+        const double be = -P.G * psi;
+#pragma unroll
+        for (int i = 0; i < 3; i++) Fi[i] = F[i] * be;
+    }
+    const double rr = rcp_rn(rho);
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        double t = Fi[j], Fx = Fi[j];
+        if (P.body) {
+            Fx += (rho - P.rho_0) * P.g[j];
+            t = Fx;
+            if (!onb) t += P.fext[j];
+        }
+        Ft[j] = t;
+        if (j >= L::D && !P.body_z) Ud[j] = 0;
+        else Ud[j] = div_rcp((j < L::D ? (double)m[j < L::D ? 3 + 2 * j : 0] : 0.0) + (L::Q == 9 ? t : Fx) * 0.5, rho, rr);
+    }
+}
+
+// The collision of a node from its moments q; f receives the populations.
+template <class L>
+__device__ __forceinline__ void collide_node32(const Params& P, const FusedArgs32& A, Pre32<L>& q, float* f, double rho,
+                                               float dr, double psi, const double* Fi, const double* Ft,
+                                               const double* Ud) {
+    const float U[3] = {(float)Ud[0], (float)Ud[1], (float)Ud[2]};
+    // conserved moments the collision must produce: the input mass, and the
+    // input momentum plus the force the collision applies
+    if constexpr (L::Q == 9) {
+        const float F[3] = {(float)Ft[0], (float)Ft[1], (float)Ft[2]};
+        const float Fv[3] = {(float)Fi[0], (float)Fi[1], (float)Fi[2]};
+        collide_limrt32(A, q.m, f, rho, dr, U, F, Fv, psi);
+#pragma unroll
+        for (int j = 0; j < L::D; j++) q.mom[j] += Ft[j];
+    } else {
+        double Fx[3];
+#pragma unroll
+        for (int j = 0; j < 3; j++) Fx[j] = P.body ? Fi[j] + (rho - P.rho_0) * P.g[j] : Fi[j];
+        const float F[3] = {(float)Fx[0], (float)Fx[1], (float)Fx[2]};
+        collide_xumrt32(A, q.m, f, rho, dr, U, F, psi);
+#pragma unroll
+        for (int j = 0; j < 3; j++) q.mom[j] += Fx[j];
+    }
+    restore_conserved<L>(f, q.mass, q.mom);
+}
+
 // After the macros: force (FP64), heat source (FP64, computed by the caller),
 // velocity, then FP32 collisions; or (EMIT) the FP64 reference state.
-template <class L, bool F_ON, bool G_ON, bool EMIT, class PsiAt>
+// LATE: the moments are evaluated after the force instead of before it.  The
+// order changes no value, only how registers are used, and which is better
+// depends on the kernel around it: with boundary programs late (97 x 61 x 83
+// walls 52 us a step, 60 early), without them early (101 x 75 x 90 periodic 52
+// us, 66 late; 2048^2 142 us, 145 late; B200).
+template <class L, bool F_ON, bool G_ON, bool EMIT, bool LATE, class PsiAt>
 __device__ __forceinline__ void finish_node32(const Params& P, const FusedArgs32& A, uint32_t id, bool onb, float* f,
                                               float* g, double rho, float dr, double T, float dT, double psi,
                                               PsiAt nbpsi, double heat, double* emit_f, double* emit_g,
                                               double* rho_out, double* Fi_out, double* Ft_out) {
     const uint32_t n = A.n;
     double Fi[3] = {0, 0, 0}, Ft[3], Ud[3];
+    Pre32<L> q;
     if constexpr (F_ON) {
-        if (!onb) {
-            double F[3] = {0.0, 0.0, 0.0};
-            static_for<L::Q - 1>([&](auto km1) {
-                constexpr int k = decltype(km1)::value + 1;
-                const double al = P.ppw[k] * nbpsi(k);
-                static_for<3>([&](auto i) {
-                    constexpr int c = ck<L>(k, decltype(i)::value);
-                    if constexpr (c == 1) F[i] += al;
-                    else if constexpr (c == -1) F[i] -= al;
-                });
-            });
-            const double be = -P.G * psi;
-#pragma unroll
-            for (int i = 0; i < 3; i++) Fi[i] = F[i] * be;
-        }
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            double t = Fi[j] + (rho - P.rho_0) * P.g[j];
-            if (!onb) t += P.fext[j];
-            Ft[j] = t;
-        }
-        // sum_k c_k f_k == sum_k c_k f~_k (sum_k c_k w_k = 0)
-        static_for<3>([&](auto jj) {
-            constexpr int j = decltype(jj)::value;
-            float lv = 0.f;
-            static_for<L::Q>([&](auto kk) {
-                constexpr int c = ck<L>(decltype(kk)::value, j);
-                if constexpr (c == 1) lv += f[kk];
-                else if constexpr (c == -1) lv -= f[kk];
-            });
-            const double Fj = L::Q == 9 ? Ft[j] : Fi[j] + (rho - P.rho_0) * P.g[j];
-            Ud[j] = ((double)lv + Fj * 0.5) / rho;
-        });
+        if constexpr (EMIT || LATE) momentum32<L>(f, q.m);
+        else pre_node32<L>(f, q);
+        force_velocity32<L>(P, onb, q.m, rho, psi, nbpsi, Fi, Ft, Ud);
     } else {
 #pragma unroll
         for (int j = 0; j < 3; j++) Ud[j] = A.Uold[(size_t)j * n + id];
@@ -512,36 +603,9 @@ __device__ __forceinline__ void finish_node32(const Params& P, const FusedArgs32
         }
         return;
     }
-    const float U[3] = {(float)Ud[0], (float)Ud[1], (float)Ud[2]};
     if constexpr (F_ON) {
-        // conserved moments the collision must produce: the input mass, and
-        // the input momentum plus the force the collision applies
-        double mass = 0.0, mom[3] = {0.0, 0.0, 0.0};
-        static_for<L::Q>([&](auto kk) {
-            constexpr int k = decltype(kk)::value;
-            mass += (double)f[k];
-            static_for<L::D>([&](auto dd) {
-                constexpr int c = ck<L>(k, decltype(dd)::value);
-                if constexpr (c == 1) mom[dd] += (double)f[k];
-                else if constexpr (c == -1) mom[dd] -= (double)f[k];
-            });
-        });
-        if constexpr (L::Q == 9) {
-            const float F[3] = {(float)Ft[0], (float)Ft[1], (float)Ft[2]};
-            const float Fv[3] = {(float)Fi[0], (float)Fi[1], (float)Fi[2]};
-            collide_limrt32(A, f, rho, dr, U, F, Fv, psi);
-#pragma unroll
-            for (int j = 0; j < 3; j++) mom[j] += Ft[j];
-        } else {
-            double Fx[3];
-#pragma unroll
-            for (int j = 0; j < 3; j++) Fx[j] = Fi[j] + (rho - P.rho_0) * P.g[j];
-            const float F[3] = {(float)Fx[0], (float)Fx[1], (float)Fx[2]};
-            collide_xumrt32(A, f, rho, dr, U, F, psi);
-#pragma unroll
-            for (int j = 0; j < 3; j++) mom[j] += Fx[j];
-        }
-        restore_conserved<L>(f, mass, mom);
+        if constexpr (LATE) pre_node32<L>(f, q);
+        collide_node32<L>(P, A, q, f, rho, dr, psi, Fi, Ft, Ud);
 #pragma unroll
         for (int k = 0; k < L::Q; k++) A.fout[(size_t)k * n + id] = f[k];
         if constexpr (G_ON) {
@@ -550,7 +614,7 @@ __device__ __forceinline__ void finish_node32(const Params& P, const FusedArgs32
         }
     }
     if constexpr (G_ON) {
-        collide_litemp32(A, g, T, dT, U[0], U[1], (float)heat);
+        collide_litemp32(A, g, T, dT, (float)Ud[0], (float)Ud[1], (float)heat);
 #pragma unroll
         for (int k = 0; k < 9; k++) A.gout[(size_t)k * n + id] = g[k];
         A.Tnew[id] = T;

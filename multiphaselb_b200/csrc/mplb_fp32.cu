@@ -5,6 +5,7 @@
 #include <algorithm>
 
 #include "fused32.cuh"
+#include "fused32_tma.cuh"
 
 namespace mplb {
 
@@ -118,7 +119,7 @@ __device__ __forceinline__ void fused32_tile_d2q9(const Params& P, const FusedAr
         }
         const double psi = F_ON ? sm.psi[ey][ex] : 0.0;
         auto nbpsi = [&](int k) { return sm.psi[ey + cyk<L>(k)][ex + cxk<L>(k)]; };
-        finish_node32<L, F_ON, G_ON, EMIT>(P, A, id, onb, f, g, rho, dr, T, dT, psi, nbpsi, heat, emit_f, emit_g,
+        finish_node32<L, F_ON, G_ON, EMIT, HAS_BC>(P, A, id, onb, f, g, rho, dr, T, dT, psi, nbpsi, heat, emit_f, emit_g,
                                            rho_out, Fi_out, Ft_out);
     }
 }
@@ -158,8 +159,11 @@ constexpr size_t f3_smem32() {
     return (size_t)3 * (TY + 2) * (TX + 2) * sizeof(double) + (size_t)2 * 15 * TX * TY * sizeof(float);
 }
 
+// The step's 32 x 4 tiles ask for five blocks per SM (at most 96 registers):
+// 101 x 75 x 90 periodic 52 us a step against 66 with four blocks of the 122
+// registers that the allocator takes otherwise (B200).
 template <int TX, int TY, bool HAS_BC, bool EMIT>
-__global__ void __launch_bounds__(TX * TY, min_blocks(TX * TY))
+__global__ void __launch_bounds__(TX * TY, !EMIT && TX * TY == 128 ? 5 : min_blocks(TX * TY))
     k_fused32_d3q15(Params P, FusedArgs32 A, double* emit_f, double* rho_out, double* Fi_out, double* Ft_out) {
     step_dependency_wait();
     using L = D3Q15T;
@@ -226,7 +230,7 @@ __global__ void __launch_bounds__(TX * TY, min_blocks(TX * TY))
 #pragma unroll
             for (int k = 0; k < 15; k++) f[k] = s_f[((z & 1) * 15 + k) * NT + tid];
             auto nbpsi = [&](int k) { return s_psi[(z + czk<L>(k) + 3) % 3][ey + cyk<L>(k)][ex + cxk<L>(k)]; };
-            finish_node32<L, true, false, EMIT>(P, A, idc, onb, f, dum, rc, drc, Tc, 0.f, s_psi[(z + 3) % 3][ey][ex],
+            finish_node32<L, true, false, EMIT, HAS_BC>(P, A, idc, onb, f, dum, rc, drc, Tc, 0.f, s_psi[(z + 3) % 3][ey][ex],
                                                 nbpsi, 0.0, emit_f, nullptr, rho_out, Fi_out, Ft_out);
         }
         __syncthreads();
@@ -256,6 +260,7 @@ FusedArgs32 mplb_make_args32(const FusedArgs& A, const Params& P, double rho_ref
     B.n = P.n;
     B.bcmap = A.bcmap;
     B.bc_margin = A.bc_margin;
+    B.kerr = A.kerr;
     for (int p = 0; p < MPLB_MAX_PATCHES; p++) B.Twall[p] = A.Twall[p];
     for (int q = 0; q < FUSED_MAX_PROGS; q++) B.prog[q] = A.prog[q];
     B.rho_ref = rho_ref;
@@ -279,9 +284,37 @@ FusedArgs32 mplb_make_args32(const FusedArgs& A, const Params& P, double rho_ref
     return B;
 }
 
+// TMA-staged 3D step: the tile for this box (-1: the general kernel takes it),
+// its extents for the tensor maps, and a launch.  64 x 8 where it divides the
+// box, else 32 x 8 at two blocks per SM (more halo per node): us per step on
+// 192^3 338 and 357 against 438 of the general kernel, on 64^3 22.4 and 22.5
+// against 27.3 (B200).
+int mplb_tma32_pick(const FusedArgs& A, bool has_bc) {
+    if (tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 64, 8)) return 0;
+    return tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 32, 8) ? 1 : -1;
+}
+void mplb_tma32_tile(int c, int* tx, int* ty) {
+    *tx = c == 0 ? 64 : 32;
+    *ty = 8;
+}
+cudaError_t mplb_tma32_launch(int c, FusedArgs32 B, const Params& P, const CUtensorMap& mf, const CUtensorMap& mT,
+                              cudaStream_t s) {
+    FusedArgs tmp{};
+    tmp.nx = B.nx; tmp.ny = B.ny; tmp.nz = B.nz;
+    const Geom g = resident_geometry(tmp, c == 0 ? 64 : 32, 8, c == 0 ? 1 : 2);
+    B.tiles_x = g.tiles_x; B.tiles_y = g.tiles_y; B.zchunk = g.zchunk;
+    if (c == 0) launch_step(k_fused32_d3q15_tma<64, 8, 1>, g.nblocks, 512, TmaTile32<64, 8>::SMEM, s, P, B, mf, mT);
+    else launch_step(k_fused32_d3q15_tma<32, 8, 2>, g.nblocks, 256, TmaTile32<32, 8>::SMEM, s, P, B, mf, mT);
+    return cudaGetLastError();
+}
+
 int mplb_fused32_attributes() {
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    chk(cudaFuncSetAttribute(k_fused32_d3q15_tma<64, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)TmaTile32<64, 8>::SMEM));
+    chk(cudaFuncSetAttribute(k_fused32_d3q15_tma<32, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)TmaTile32<32, 8>::SMEM));
     chk(set32<32, 8, true, true>());
     chk(set32<32, 8, false, true>());
     chk(set32<32, 4, true, false>());
