@@ -356,27 +356,15 @@ inline bool fused_supported(int lat, const int* model, const Params& P, const st
     return true;
 }
 
-inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params& P, const std::vector<PatchDev>* fp,
-                       const mplb_mesh_desc* mesh, const int* dims, const int* per, cudaStream_t stream,
-                       uint64_t* bytes) {
-    (void)model;
-    FusedArgs& A = fc.args;
-    A.nx = dims[0];
-    A.ny = dims[1];
-    A.nz = lat == MPLB_D3Q15 ? dims[2] : 1;
-    A.px = per[0];
-    A.py = per[1];
-    A.pz = lat == MPLB_D3Q15 ? per[2] : 1;
-    A.own_lo = 0;
-    A.own_cnt = P.n;  // every node's outputs stored; slabs narrow it (mplb_gpu_set_owned)
-    A.nmirror = 0;
+// The boundary program of every node (index into progs; 0 = none).
+inline int node_programs(const Params& P, const std::vector<PatchDev>* fp, const mplb_mesh_desc* mesh,
+                         std::vector<uint8_t>& map, std::vector<BCProg>& progs, bool& any, std::string& err) {
     // Node programs: for every node, the ops of every patch holding it, in
     // patch order, per field.  Identical programs share one table entry.
     const uint32_t n = P.n;
-    std::vector<uint8_t> map(n, 0);
-    std::vector<BCProg> progs(1, BCProg{});
-    std::vector<BCProg> per_node;
-    bool any = false;
+    map.assign(n, 0);
+    progs.assign(1, BCProg{});
+    any = false;
     {
         std::vector<BCProg> node(n, BCProg{});
         size_t off = 0;
@@ -389,10 +377,10 @@ inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params&
                     if (t != MPLB_BC_BOUNCEBACK && t != MPLB_BC_FIXEDT) continue;
                     BCProg& b = node[id];
                     if (fi == 0) {
-                        if (b.nf >= FUSED_MAX_OPS) { fc.err = "too many boundary ops on one node"; return MPLB_E_UNSUPPORTED; }
+                        if (b.nf >= FUSED_MAX_OPS) { err = "too many boundary ops on one node"; return MPLB_E_UNSUPPORTED; }
                         b.ft[b.nf++] = (uint8_t)t;
                     } else {
-                        if (b.ng >= FUSED_MAX_OPS) { fc.err = "too many boundary ops on one node"; return MPLB_E_UNSUPPORTED; }
+                        if (b.ng >= FUSED_MAX_OPS) { err = "too many boundary ops on one node"; return MPLB_E_UNSUPPORTED; }
                         b.gp[b.ng] = (uint8_t)p;
                         b.gt[b.ng++] = (uint8_t)t;
                     }
@@ -408,13 +396,35 @@ inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params&
             for (size_t q = 1; q < progs.size(); q++)
                 if (std::memcmp(&progs[q], &b, sizeof(BCProg)) == 0) { found = (int)q; break; }
             if (found < 0) {
-                if (progs.size() >= FUSED_MAX_PROGS) { fc.err = "too many distinct boundary programs"; return MPLB_E_UNSUPPORTED; }
+                if (progs.size() >= FUSED_MAX_PROGS) { err = "too many distinct boundary programs"; return MPLB_E_UNSUPPORTED; }
                 progs.push_back(b);
                 found = (int)progs.size() - 1;
             }
             map[id] = (uint8_t)found;
         }
     }
+    return 0;
+}
+
+inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params& P, const std::vector<PatchDev>* fp,
+                       const mplb_mesh_desc* mesh, const int* dims, const int* per, cudaStream_t stream,
+                       uint64_t* bytes) {
+    (void)model;
+    FusedArgs& A = fc.args;
+    A.nx = dims[0];
+    A.ny = dims[1];
+    A.nz = lat == MPLB_D3Q15 ? dims[2] : 1;
+    A.px = per[0];
+    A.py = per[1];
+    A.pz = lat == MPLB_D3Q15 ? per[2] : 1;
+    A.own_lo = 0;
+    A.own_cnt = P.n;  // every node's outputs stored; slabs narrow it (mplb_gpu_set_owned)
+    A.nmirror = 0;
+    std::vector<uint8_t> map;
+    std::vector<BCProg> progs;
+    bool any = false;
+    if (int rc = node_programs(P, fp, mesh, map, progs, any, fc.err)) return rc;
+    const uint32_t n = P.n;
     // farthest distance of a node with a boundary program from its nearest
     // box face (-1: none); tiles whose ring lies farther in hold none
     A.bc_margin = -1;

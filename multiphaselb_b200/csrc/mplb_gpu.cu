@@ -21,8 +21,12 @@
 #include "ops.cuh"
 #include "fused_host.cuh"
 #include "fused32.cuh"
+#include "fused_table.cuh"
 
 using namespace mplb;
+
+// Fused steps on neighbour tables (mplb_table.cu).
+int mplb_table_step(int lat, int heat, bool emit, bool st, const Params& P, const TableArgs& A, cudaStream_t s);
 
 // FP32-deviation kernels (mplb_fp32.cu, compiled with contraction on).
 FusedArgs32 mplb_make_args32(const FusedArgs& A, const Params& P, double rho_ref, double T_ref);
@@ -162,6 +166,10 @@ struct mplb_gpu {
     } mirrors[MPLB_MAX_MIRRORS] = {};
     int nmirror = 0;
     cudaEvent_t order_ev = nullptr;
+    // operator path: mplb_gpu_step runs the fused kernels of fused_table.cuh where
+    // they take this lattice (their buffers are made at the first such step)
+    bool table = false;
+    TableArgs tab{};
     uint64_t launches = 0;
     uint64_t bytes = 0;
     bool initialized = false;
@@ -192,6 +200,8 @@ void free_all(mplb_gpu* h) {
             if (h->p32[i][j]) cudaFree(h->p32[i][j]);
     if (h->snap) cudaFree(h->snap);
     if (h->mom) cudaFree(h->mom);
+    if (h->tab.psi) cudaFree(h->tab.psi);
+    if (h->tab.bcmap) cudaFree(const_cast<uint8_t*>(h->tab.bcmap));
     for (int i = 0; i < 2; i++)
         if (h->bctab[i]) cudaFree(h->bctab[i]);
 }
@@ -928,6 +938,101 @@ int enter_fused(mplb_gpu* h) {
     return 0;
 }
 
+// Operator path: can mplb_gpu_step run the kernels of fused_table.cuh?  They
+// take an updated flow and boundary patches that need only a node's own
+// populations, or, for fixedT, an inner neighbour's that no other op writes.
+int table_setup(mplb_gpu* h, const mplb_mesh_desc* mesh) {
+    if (h->precision != MPLB_FP64 || !h->P.f_update || h->serial[0] || h->serial[1]) return 0;
+    for (int fi = 0; fi < 2; fi++) {
+        if (!(fi == 0 ? h->P.f_update : h->P.g_update)) continue;
+        for (const PatchDev& pt : h->fpatch[fi])
+            if (pt.type != MPLB_BC_PERIODIC && pt.type != MPLB_BC_BOUNCEBACK && !(pt.type == MPLB_BC_FIXEDT && fi == 1) &&
+                !(pt.type == MPLB_BC_FIXEDU && h->model[fi] != MPLB_LIMRT))
+                return 0;
+    }
+    std::vector<uint8_t> map;
+    std::vector<BCProg> progs;
+    std::string why;
+    bool any = false;
+    if (node_programs(h->P, h->fpatch, mesh, map, progs, any, why)) return 0;
+    if (any) {
+        uint8_t* m = nullptr;
+        RET(dalloc(h, &m, h->n));
+        h->tab.bcmap = m;
+        CK(cudaMemcpyAsync(m, map.data(), h->n, cudaMemcpyHostToDevice, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+    }
+    for (size_t q = 0; q < progs.size(); q++) h->tab.prog[q] = progs[q];
+    for (size_t p = 0; p < h->fpatch[1].size() && p < MPLB_MAX_PATCHES; p++) h->tab.Twall[p] = h->fpatch[1][p].val[0];
+    h->table = true;
+    return 0;
+}
+
+// One step of fused_table.cuh, or (emit) the reference state after the last one.
+int table_step(mplb_gpu* h, bool emit) {
+    const bool gon = h->P.g_update != 0;
+    const int heat = !gon ? TABLE_NONE : (h->model[1] == MPLB_MYMRT ? TABLE_MY : TABLE_LITEMP);
+    TableArgs A = h->tab;
+    A.nb = h->nb;
+    A.onb = h->onb;
+    const int c0 = h->cur[0], c1 = h->cur[1], e = emit ? 1 : 0;
+    A.fin = h->pdf[0][c0 ^ e];
+    A.fout = h->pdf[0][c0 ^ e ^ 1];
+    A.gin = gon ? h->pdf[1][c1 ^ e] : nullptr;
+    A.gout = gon ? h->pdf[1][c1 ^ e ^ 1] : nullptr;
+    A.Told = gon && emit ? h->T2 : h->T;
+    A.Tnew = gon ? h->T2 : nullptr;
+    A.Uold = gon && emit ? h->U2 : h->U;
+    A.Unew = gon && !emit ? h->U2 : h->U;
+    A.S = h->S;
+    A.rho = h->rho;
+    A.Fi = h->Fi;
+    A.Ft = h->Ft;
+    h->launches += mplb_table_step(h->lat, heat, emit, h->P.st_on != 0, h->P, A, h->stream);
+    RET(launch_check(h));
+    if (!emit) {
+        h->cur[0] ^= 1;
+        if (gon) {
+            h->cur[1] ^= 1;
+            std::swap(h->T, h->T2);
+            std::swap(h->U, h->U2);
+        }
+    }
+    return 0;
+}
+
+// Enter the fused state.  Without memory for the kernels' buffers the lattice
+// stays on the operators.
+int table_enter(mplb_gpu* h) {
+    if (!h->tab.psi) {
+        const bool gon = h->P.g_update != 0;
+        double* buf[3] = {nullptr, nullptr, nullptr};
+        const size_t count[3] = {2 * (size_t)h->n, gon ? (size_t)h->n : 0, gon ? 3 * (size_t)h->n : 0};
+        for (int i = 0; i < 3; i++) {
+            if (!count[i] || cudaMalloc((void**)&buf[i], count[i] * sizeof(double)) == cudaSuccess) continue;
+            cudaGetLastError();
+            for (double* b : buf) cudaFree(b);
+            h->table = false;
+            return 0;
+        }
+        for (int i = 0; i < 3; i++) {
+            if (!buf[i]) continue;
+            h->bytes += count[i] * sizeof(double);
+            CK(cudaMemsetAsync(buf[i], 0, count[i] * sizeof(double), h->stream));
+        }
+        h->tab.psi = buf[0];
+        h->tab.inv = buf[0] + h->n;
+        h->T2 = buf[1];
+        h->U2 = buf[2];
+    }
+    if (h->fstate == 0) {
+        RET(DISPATCH(h, op_collision, h, 0));
+        RET(DISPATCH(h, op_collision, h, 1));
+        h->fstate = 1;
+    }
+    return 0;
+}
+
 // One strided node copy: `rows` component rows of a [component][node] array.
 struct NodeCopy {
     double* d;
@@ -939,7 +1044,8 @@ int copy_node_rows(mplb_gpu* dst, uint32_t dst_start, mplb_gpu* src, uint32_t sr
 
 int materialize(mplb_gpu* h) {
     if (h->fstate == 0) return 0;
-    if (h->precision == MPLB_FP32_DEV) RET(fused32_step(h, true));
+    if (h->path == MPLB_PATH_OPERATORS) RET(table_step(h, true));
+    else if (h->precision == MPLB_FP32_DEV) RET(fused32_step(h, true));
     else RET(fused_step(h, true));
     h->fstate = 0;
     return 0;
@@ -1227,6 +1333,7 @@ int mplb_gpu_create(const mplb_mesh_desc* mesh, const mplb_eos_desc* eos, const 
             if (mplb_fused32_attributes()) return bail(fail(MPLB_E_CUDA, "cannot raise the shared memory limit (FP32 kernels)"));
         }
     }
+    else if ((rc = table_setup(h, mesh))) return bail(rc);
     h->red_parts = 2 * 148;
     if ((rc = dalloc(h, &h->red, 2 * (size_t)h->red_parts + 8))) return bail(rc);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bail(fail(MPLB_E_CUDA, "device set-up failed"));
@@ -1335,6 +1442,12 @@ int mplb_gpu_step(mplb_gpu_t* h, uint32_t nsteps) {
                                       "step in between)");
         RET(enter_fused(h));  // prologue: the first collision of the loop, on the reference state
         for (uint32_t s = 0; s < nsteps; s++) RET(fused_step(h, false));
+        h->current += nsteps;
+        return 0;
+    }
+    if (h->table) RET(table_enter(h));
+    if (h->table) {
+        for (uint32_t s = 0; s < nsteps; s++) RET(table_step(h, false));
         h->current += nsteps;
         return 0;
     }
@@ -1607,6 +1720,8 @@ int mplb_gpu_monitor(mplb_gpu_t* h, int32_t reset, double* max_drho, double* mas
         k_monitor_partial<float><<<parts, TPB, 0, h->stream>>>(h->n, h->Q, h->p32[0][h->cur32[0]], h->rho_ref,
                                                                h->snap, reset, h->red);
     } else {
+        // on the operator path the sum is macroDensity's, of the streamed populations
+        if (h->path == MPLB_PATH_OPERATORS) RET(materialize(h));
         if (h->path == MPLB_PATH_FUSED && h->fstate == 0) {
             RET(DISPATCH(h, op_collision, h, 0));
             RET(DISPATCH(h, op_collision, h, 1));
