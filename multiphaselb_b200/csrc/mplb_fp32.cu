@@ -25,7 +25,9 @@ struct Smem32 {
 // INNER: the tile, its ring and the ring's pull sources lie inside the box
 // and away from every boundary program (see the FP64 kernel), so the wrap /
 // missing-source / boundary bookkeeping is skipped.
-template <int TX, int TY, bool F_ON, bool G_ON, bool HAS_BC, bool EMIT, bool INNER = false>
+// RINGW: added warps that compute the ring, one slot per thread (see the FP64
+// kernel); 0: the node threads compute it first.
+template <int TX, int TY, bool F_ON, bool G_ON, bool HAS_BC, bool EMIT, bool INNER = false, int RINGW = 0>
 __device__ __forceinline__ void fused32_tile_d2q9(const Params& P, const FusedArgs32& A, Smem32<TX, TY, G_ON>& sm,
                                                   int bx, int by, double* emit_f, double* emit_g, double* rho_out,
                                                   double* Fi_out, double* Ft_out) {
@@ -70,22 +72,33 @@ __device__ __forceinline__ void fused32_tile_d2q9(const Params& P, const FusedAr
         const int px = x0 + tx, py = y0 + ty;
         prefetch_node32<L, F_ON, G_ON>(A, px, py, (uint32_t)px + (uint32_t)A.nx * (uint32_t)py);
     }
-    for (int r = threadIdx.x; r < NRING; r += blockDim.x) {
-        int ex, ey;
-        ring_slot(r, TX, TY, ex, ey);
-        float rf[9], rg[9], rdr, rdt;
-        double rrho, rt, rrr;
-        EosRho rer;
-        uint32_t rid;
-        slot(ex, ey, rf, rg, rrho, rt, rdr, rdt, rid, false, rrr, rer);
+    if constexpr (RINGW == 0) {
+        for (int r = threadIdx.x; r < NRING; r += blockDim.x) {
+            int ex, ey;
+            ring_slot(r, TX, TY, ex, ey);
+            float rf[9], rg[9], rdr, rdt;
+            double rrho, rt, rrr;
+            EosRho rer;
+            uint32_t rid;
+            slot(ex, ey, rf, rg, rrho, rt, rdr, rdt, rid, false, rrr, rer);
+        }
     }
     float f[9], g[9], dr = 0.f, dT = 0.f;
     double rho = 0, T = 0, rr = 0;
     EosRho er{};
     uint32_t id = 0;
     const int gx = x0 + tx, gy = y0 + ty;
-    const bool own = INNER || (gx < A.nx && gy < A.ny);
-    const bool have = slot(tx + 1, ty + 1, f, g, rho, T, dr, dT, id, own, rr, er);
+    static_assert(RINGW == 0 || NRING <= 32 * RINGW, "one ring slot per ring thread");
+    const bool ringer = RINGW > 0 && (int)threadIdx.x >= TX * TY;
+    const bool own = !ringer && (INNER || (gx < A.nx && gy < A.ny));
+    int sx = tx + 1, sy = ty + 1;
+    bool act = true;
+    if (ringer) {
+        const int r = (int)threadIdx.x - TX * TY;
+        act = r < NRING;
+        if (act) ring_slot(r, TX, TY, sx, sy);
+    }
+    const bool have = act && slot(sx, sy, f, g, rho, T, dr, dT, id, own, rr, er);
     __syncthreads();
     if (own && have) {
         const int ex = tx + 1, ey = ty + 1;
@@ -128,8 +141,9 @@ __device__ __forceinline__ void fused32_tile_d2q9(const Params& P, const FusedAr
 // MINB: resident blocks per SM asked of the register allocator (0 = default).
 // TRY_INNER: inner tiles take the lean body (large lattices); otherwise the
 // kernel holds the general body alone (a lattice of one wave prefers it).
-template <int TX, int TY, bool F_ON, bool G_ON, bool HAS_BC, bool EMIT, int MINB = 0, bool TRY_INNER = false>
-__global__ void __launch_bounds__(TX * TY, MINB ? MINB : min_blocks(TX * TY))
+// RINGW: added warps that compute the ring.
+template <int TX, int TY, bool F_ON, bool G_ON, bool HAS_BC, bool EMIT, int MINB = 0, bool TRY_INNER = false, int RINGW = 0>
+__global__ void __launch_bounds__(TX * TY + 32 * RINGW, MINB ? MINB : min_blocks(TX * TY))
     k_fused32_d2q9(Params P, FusedArgs32 A, double* emit_f, double* emit_g, double* rho_out, double* Fi_out,
                    double* Ft_out) {
     step_dependency_wait();
@@ -144,14 +158,21 @@ __global__ void __launch_bounds__(TX * TY, MINB ? MINB : min_blocks(TX * TY))
             return;
         }
     }
-    fused32_tile_d2q9<TX, TY, F_ON, G_ON, HAS_BC, EMIT, false>(P, A, sm, bx, by, emit_f, emit_g, rho_out, Fi_out,
-                                                               Ft_out);
+    fused32_tile_d2q9<TX, TY, F_ON, G_ON, HAS_BC, EMIT, false, RINGW>(P, A, sm, bx, by, emit_f, emit_g, rho_out,
+                                                                      Fi_out, Ft_out);
 }
 
-// Lattices of more tiles than this (32 x 8) take the register-capped
-// inner-tile kernel: several waves, where it measured faster; fewer (one
-// wave or so) keep the general kernel.
-constexpr int F32_INNER_MIN_TILES = 4 * 148;
+// Which 2D kernel steps a lattice, by its tiles of 32 x 8 (us a step, B200):
+//   * up to seven per SM: tiles with ring warps, so that every thread has one slot
+//     to fill before the barrier.  16 x 8 + 2 warps, four blocks per SM (64^2 3.2,
+//     192^2 3.6, 512^2 9.9, thermal 64 x 256 5.8), or, where 32 x 8 + 3 warps at
+//     two blocks per SM just fill the device, those (256^2 4.0 against 4.6,
+//     thermal 128 x 512 7.5 against 7.7, 128 x 256 6.1 against 6.4); without ring
+//     warps 64^2 3.9, 256^2 4.6, 128 x 512 9.0.
+//   * more: 16 x 8 tiles at eight blocks per SM (64 registers), inner tiles lean
+//     (517 x 733 13.7, 2048^2 118, thermal 512 x 1024 39, 1024 x 4096 231; the
+//     ring-warp tiles 14.5, 137, 43, 297; 32 x 8 at three blocks 15.5, 142, -, 250).
+constexpr int F32_CAPPED_MIN_TILES = 7 * 148;
 
 // ------------------------------------------------------------- 3D kernel
 template <int TX, int TY>
@@ -327,26 +348,26 @@ cudaError_t mplb_fused32_launch(int lat, bool has_bc, bool f_on, bool g_on, bool
                                 const Params& P, double* emit_f, double* emit_g, double* rho_out, double* Fi_out,
                                 double* Ft_out, cudaStream_t s) {
     if (lat == MPLB_D2Q9) {
-        FusedArgs tmp{};
-        tmp.nx = B.nx; tmp.ny = B.ny; tmp.nz = 1;
-        const Geom g = fused_geometry(MPLB_D2Q9, tmp, 32, 8);
-        B.tiles_x = g.tiles_x;
-        B.tiles_y = g.tiles_y;
-        B.zchunk = 1;
-        const bool big = !emit && g.nblocks > F32_INNER_MIN_TILES;
-#define MPLB_L32(F, G, BC, E)                                                                              \
-    (big ? (launch_step(k_fused32_d2q9<32, 8, F, G, BC, E, 3, true>, g.nblocks, 256, 0, s, P, B, emit_f, emit_g, \
-                        rho_out, Fi_out, Ft_out), 0)                                                              \
-         : (launch_step(k_fused32_d2q9<32, 8, F, G, BC, E>, g.nblocks, 256, 0, s, P, B, emit_f, emit_g, rho_out,  \
-                        Fi_out, Ft_out), 0))
-#define MPLB_L32_E(F, G, BC) (emit ? (MPLB_L32(F, G, BC, true), 0) : (MPLB_L32(F, G, BC, false), 0))
-#define MPLB_L32_B(F, G) (has_bc ? MPLB_L32_E(F, G, true) : MPLB_L32_E(F, G, false))
-        if (f_on && g_on) MPLB_L32_B(true, true);
-        else if (f_on) MPLB_L32_B(true, false);
-        else if (g_on) MPLB_L32_B(false, true);
-#undef MPLB_L32
-#undef MPLB_L32_E
-#undef MPLB_L32_B
+        auto go = [&](auto kern, int tx, int ty, int nt) {
+            B.tiles_x = (B.nx + tx - 1) / tx;
+            B.tiles_y = (B.ny + ty - 1) / ty;
+            B.zchunk = 1;
+            launch_step(kern, B.tiles_x * B.tiles_y, nt, 0, s, P, B, emit_f, emit_g, rho_out, Fi_out, Ft_out);
+        };
+        auto pick = [&](auto F, auto G, auto BC) {
+            constexpr bool f = decltype(F)::value, g = decltype(G)::value, bc = decltype(BC)::value;
+            if (emit) return go(k_fused32_d2q9<32, 8, f, g, bc, true>, 32, 8, 256);
+            const int tiles = ((B.nx + 31) / 32) * ((B.ny + 7) / 8);
+            if (tiles > F32_CAPPED_MIN_TILES) return go(k_fused32_d2q9<16, 8, f, g, bc, false, 8, true>, 16, 8, 128);
+            if (tiles > (g ? 74 : 148) && tiles <= 2 * 148)
+                return go(k_fused32_d2q9<32, 8, f, g, bc, false, 2, false, 3>, 32, 8, 352);
+            return go(k_fused32_d2q9<16, 8, f, g, bc, false, 4, false, 2>, 16, 8, 192);
+        };
+        using std::true_type;
+        using std::false_type;
+        if (f_on && g_on) has_bc ? pick(true_type{}, true_type{}, true_type{}) : pick(true_type{}, true_type{}, false_type{});
+        else if (f_on) has_bc ? pick(true_type{}, false_type{}, true_type{}) : pick(true_type{}, false_type{}, false_type{});
+        else if (g_on) has_bc ? pick(false_type{}, true_type{}, true_type{}) : pick(false_type{}, true_type{}, false_type{});
     } else {
         FusedArgs tmp{};
         tmp.nx = B.nx; tmp.ny = B.ny; tmp.nz = B.nz;
@@ -394,9 +415,10 @@ constexpr int N_BATCH_CFG = 4;
 constexpr TileCfg BATCH_CFG[N_BATCH_CFG] = {{32, 8, false}, {32, 4, false}, {16, 8, false}, {64, 4, false}};
 
 // The batch fills every SM with a persistent grid, so resident warps hide
-// its memory latency: registers are capped for 24 warps per SM (3 blocks of
-// 256 threads, 6 of 128) instead of the lone kernel's 16.
-constexpr int batch_min_blocks(int threads) { return threads <= 128 ? 6 : 3; }
+// its memory latency: registers are capped for 32 warps per SM (4 blocks of
+// 256 threads, 8 of 128; a few spills), 63.5 us a step of a 24-bubble ensemble
+// against 67.5 with 24 warps (B200).
+constexpr int batch_min_blocks(int threads) { return threads <= 128 ? 8 : 4; }
 
 template <int TX, int TY>
 __global__ void __launch_bounds__(TX * TY, batch_min_blocks(TX * TY))

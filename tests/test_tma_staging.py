@@ -46,3 +46,27 @@ def test_fp32_3d_steps(gpu_lib, dims):
         got = lat.download()
     assert np.linalg.norm(got["rho"] - want["rho"]) <= 5e-7 * np.linalg.norm(want["rho"])
     assert np.abs(got["U"] - want["U"]).max() <= 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [(16, 8), (24, 20), (96, 64), (256, 256), (300, 290), (512, 530)])
+@pytest.mark.parametrize("heat", [False, True])
+def test_fp32_2d_steps(gpu_lib, dims, heat):
+    """The sizes at which the FP32 2D step changes its kernel (tiles of 32 x 8 up to
+    74, 148, 296, 1036 and more), partial tiles among them, in six steps against
+    the FP64 oracle; bounds as for the 3D steps (densities 0.02 and more)."""
+    from multiphaselb_b200 import Lattice
+    if heat:
+        case = cases.perturbed(cases.column_case(*dims, amp=1e-3, width=3.0), du=1e-3)
+    else:
+        case = cases.perturbed(cases.bubble_case(abi.D2Q9, 8, 2.5, 3.0, 0.8, dims=dims), du=1e-3)
+    want = run_checker("port", case, 6)
+    with Lattice(case, path=abi.PATH_FUSED, precision=abi.FP32_DEV) as lat:
+        lat.upload_case()
+        lat.initialize()
+        lat.step(4)
+        lat.step(2)
+        got = lat.download()
+    for k in ("rho", "T"):
+        assert np.linalg.norm(got[k] - want[k]) <= 5e-7 * np.linalg.norm(want[k]), k
+    assert np.abs(got["U"] - want["U"]).max() <= 1e-5
