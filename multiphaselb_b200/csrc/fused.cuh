@@ -968,6 +968,7 @@ struct TileCfg {
     bool tma;    // 3D only: planes staged by TMA (k_fused_d3q15_tma; fully periodic boxes)
     int ringw;   // 2D only: added warps that compute the ring (k_fused_d2q9 RINGW)
     bool march;  // 2D myMRT heat only: the marching kernel (k_march_my_d2q9)
+    bool table;  // 3D only: the kernels on the neighbour table (fused_table.cuh)
 };
 constexpr int N_CFG2 = 11, N_CFG3 = 10, N_CFG_MAX = 11;
 constexpr TileCfg CFG2[N_CFG2] = {{32, 8, false, 0, false}, {32, 4, false, 0, false}, {64, 4, false, 0, false},
@@ -976,7 +977,8 @@ constexpr TileCfg CFG2[N_CFG2] = {{32, 8, false, 0, false}, {32, 4, false, 0, fa
                                   {32, 8, false, 2, false, false, 3}, {16, 8, false, 4, false, false, 2},
                                   {28, 1, false, 0, false, false, 0, true}};
 constexpr TileCfg CFG3[N_CFG3] = {{32, 8, false, 0, false}, {32, 8, true, 0, false}, {32, 4, false, 0, false},
-                                  {64, 4, false, 0, false}, {32, 16, false, 0, false}, {64, 8, false, 0, false},
+                                  {64, 4, false, 0, false}, {32, 16, false, 0, false},
+                                  {32, 4, false, 0, false, false, 0, false, true},
                                   {32, 4, false, 3, false, true}, {32, 8, false, 2, false, true},
                                   {32, 16, false, 1, false, true}, {64, 8, false, 1, false, true}};
 

@@ -8,11 +8,16 @@
 
 #include "fused.cuh"
 #include "fused_march.cuh"
+#include "fused_table.cuh"
 #include "fused_tma.cuh"
 
 // The marching D2Q9 step with myMRT heat (mplb_march.cu).
 int mplb_march_resident(bool f_on, bool bc);
 cudaError_t mplb_march_launch(bool f_on, bool bc, int nb, const mplb::Params& P, const mplb::FusedArgs& A, cudaStream_t s);
+
+// Steps on neighbour tables (mplb_table.cu); returns the launches made.
+int mplb_table_step(int lat, int heat, bool emit, bool st, const mplb::Params& P, const mplb::TableArgs& A,
+                    cudaStream_t s);
 
 namespace mplb {
 
@@ -39,6 +44,10 @@ struct FusedConfig {
     int ncfg = 0;
     int nblocks = 0;
     double* my_scratch = nullptr;  // myMRT: rho_a and gsum_a, 2 n doubles
+    // table candidate (D3Q15): table, flags and scratch; the
+    // best tile candidate, which takes the steps of slabs (owned and mirrored ranges)
+    TableArgs tab{};
+    int tile_cfg = 2;
     int* kerr = nullptr;           // kernel error flag (bounded waits), one int
     int* kerr_host = nullptr;      // its pinned host copy
     TmaMaps tmaps[4];              // two TMA candidates x two population buffers
@@ -121,7 +130,6 @@ inline cudaError_t fused_attributes() {
     MPLB_SET3(32, 4, false)
     MPLB_SET3(64, 4, false)
     MPLB_SET3(32, 16, false)
-    MPLB_SET3(64, 8, false)
 #undef MPLB_SET3
 #define MPLB_SET3_TMA(TX, TY, MINB)                                                                                          \
     chk(cudaFuncSetAttribute(k_fused_d3q15_tma<TX, TY, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
@@ -193,6 +201,20 @@ void launch3(bool bc, int nb, const Params& P, const FusedArgs& A, cudaStream_t 
 // Launch one fused step with candidate `cfg` (EMIT always uses candidate 0).
 inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, FusedArgs A, bool f_on, bool g_on,
                                     bool emit, cudaStream_t s) {
+    if (fc.lat == MPLB_D3Q15 && CFG3[cfg].table && !emit && fc.geom[cfg].nblocks) {
+        if (A.own_cnt == P.n && !A.nmirror) {
+            TableArgs T = fc.tab;
+            T.fin = A.fin;
+            T.fout = A.fout;
+            T.Told = A.Told;
+            T.Uold = A.Uold;
+            T.Unew = A.Unew;
+            T.rho = A.rho_out;  // rewritten with the reference state
+            mplb_table_step(fc.lat, TABLE_NONE, false, P.st_on != 0, P, T, s);
+            return cudaGetLastError();
+        }
+        cfg = fc.tile_cfg;
+    }
     // surface tension: one tile shape per kernel family stands for all candidates
     const bool st = P.st_on && f_on && !emit;
     const bool tma = fc.lat == MPLB_D3Q15 && CFG3[cfg].tma;
@@ -234,7 +256,6 @@ inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, F
             case 2: launch3<32, 4, false, false>(bc, nb, P, A, s); break;
             case 3: launch3<64, 4, false, false>(bc, nb, P, A, s); break;
             case 4: launch3<32, 16, false, false>(bc, nb, P, A, s); break;
-            case 5: launch3<64, 8, false, false>(bc, nb, P, A, s); break;
             case 6: if (cudaError_t e = launch3_tma<32, 4, 3>(fc, cfg, nb, P, A, s)) return e; break;
             case 7: if (cudaError_t e = launch3_tma<32, 8, 2>(fc, cfg, nb, P, A, s)) return e; break;
             case 8: if (cudaError_t e = launch3_tma<32, 16, 1>(fc, cfg, nb, P, A, s)) return e; break;
@@ -319,6 +340,14 @@ inline int fused_autotune(FusedConfig& fc, const Params& P, const FusedArgs& A, 
             best = med;
             best_cfg = c;
         }
+    }
+    if (fc.lat == MPLB_D3Q15) {
+        best = 1e30f;
+        for (int c = 0; c < fc.ncfg; c++)
+            if (!CFG3[c].table && ok_c[c] && fc.tune_ms[c] < best) {
+                best = fc.tune_ms[c];
+                fc.tile_cfg = c;
+            }
     }
     cudaGetLastError();
     for (int i = 0; i < TIMED + 1; i++) cudaEventDestroy(ev[i]);
@@ -407,9 +436,8 @@ inline int node_programs(const Params& P, const std::vector<PatchDev>* fp, const
 }
 
 inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params& P, const std::vector<PatchDev>* fp,
-                       const mplb_mesh_desc* mesh, const int* dims, const int* per, cudaStream_t stream,
-                       uint64_t* bytes) {
-    (void)model;
+                       const mplb_mesh_desc* mesh, const int* dims, const int* per, const int32_t* nb,
+                       const uint8_t* onb, cudaStream_t stream, uint64_t* bytes) {
     FusedArgs& A = fc.args;
     A.nx = dims[0];
     A.ny = dims[1];
@@ -477,6 +505,22 @@ inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params&
         const TileCfg t = lat == MPLB_D2Q9 ? CFG2[c] : CFG3[c];
         if (t.tma) {
             fc.geom[c] = tma3_fits(A, any, t.tx, t.ty) ? resident_geometry(A, t.tx, t.ty, t.minb) : Geom{0, 0, 0, 0};
+        } else if (t.table) {
+            // two kernels that pull twice but have no ring, barrier or wrap arithmetic:
+            // the better ones where boundary programs make a pull costly (us a step,
+            // walls 97 x 61 x 83: 69 against 88 of the best tile; periodic 101 x 75 x
+            // 90: 94 against 86; B200).  Offered if the scratch, a double a node, can be had.
+            fc.geom[c] = Geom{0, 0, 0, 0};
+            if (cudaMalloc((void**)&fc.tab.psi, (size_t)n * sizeof(double)) == cudaSuccess) {
+                *bytes += (size_t)n * sizeof(double);
+                fc.tab.nb = nb;
+                fc.tab.onb = onb;
+                fc.tab.bcmap = fc.bcmap;
+                for (int q = 0; q < FUSED_MAX_PROGS; q++) fc.tab.prog[q] = A.prog[q];
+                fc.geom[c] = Geom{1, 1, 1, (int)((n + 127) / 128)};
+            } else {
+                cudaGetLastError();
+            }
         } else if (t.march) {
             const bool my = P.g_update && model[1] == MPLB_MYMRT;
             fc.geom[c] = my ? march_geometry(A, mplb_march_resident(P.f_update != 0, any)) : Geom{0, 0, 0, 0};
@@ -519,6 +563,8 @@ inline void fused_free(FusedConfig& fc) {
     fc.bcmap = nullptr;
     if (fc.my_scratch) cudaFree(fc.my_scratch);
     fc.my_scratch = nullptr;
+    if (fc.tab.psi) cudaFree(fc.tab.psi);
+    fc.tab.psi = nullptr;
 }
 
 

@@ -137,7 +137,7 @@ __device__ __forceinline__ void table_gradients(const TableArgs& A, uint32_t n, 
 }
 
 template <class L, int GM>
-__global__ void __launch_bounds__(128, L::Q == 9 ? 8 : 4) k_table_sum(Params P, TableArgs A) {
+__global__ void __launch_bounds__(128, L::Q == 9 || GM == TABLE_NONE ? 8 : 4) k_table_sum(Params P, TableArgs A) {
     step_dependency_wait();
     const uint32_t n = P.n, id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(128) k_table_heat(Params P, TableArgs A) {
 }
 
 template <class L, int GM, bool EMIT, bool ST>
-__global__ void __launch_bounds__(128, L::Q == 9 ? 6 : 3) k_table_finish(Params P, TableArgs A) {
+__global__ void __launch_bounds__(128, L::Q == 9 ? 6 : (GM == TABLE_NONE ? 5 : 3)) k_table_finish(Params P, TableArgs A) {
     step_dependency_wait();
     const uint32_t n = P.n, id = blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= n) return;

@@ -25,8 +25,6 @@
 
 using namespace mplb;
 
-// Fused steps on neighbour tables (mplb_table.cu).
-int mplb_table_step(int lat, int heat, bool emit, bool st, const Params& P, const TableArgs& A, cudaStream_t s);
 
 // FP32-deviation kernels (mplb_fp32.cu, compiled with contraction on).
 FusedArgs32 mplb_make_args32(const FusedArgs& A, const Params& P, double rho_ref, double T_ref);
@@ -1322,7 +1320,7 @@ int mplb_gpu_create(const mplb_mesh_desc* mesh, const mplb_eos_desc* eos, const 
         return bail(fail(MPLB_E_UNSUPPORTED, "FP32-deviation storage runs on the fused path only"));
     h->path = (want_path == MPLB_PATH_OPERATORS || !fusable) ? MPLB_PATH_OPERATORS : MPLB_PATH_FUSED;
     if (h->path == MPLB_PATH_FUSED) {
-        if ((rc = fused_setup(h->fc, h->lat, h->model, h->P, h->fpatch, mesh, h->dims, h->per, h->stream, &h->bytes)))
+        if ((rc = fused_setup(h->fc, h->lat, h->model, h->P, h->fpatch, mesh, h->dims, h->per, h->nb, h->onb, h->stream, &h->bytes)))
             return bail(fail(rc, "fused setup: " + h->fc.err));
         if ((rc = dalloc(h, &h->T2, h->n)) || (rc = dalloc(h, &h->U2, 3 * (size_t)h->n))) return bail(rc);
         if (h->precision == MPLB_FP32_DEV) {

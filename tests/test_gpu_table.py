@@ -59,3 +59,21 @@ def test_launches_per_step(gpu_lib, name, fused):
         lat.step(10)
         per_step = (lat.info()["kernel_launches"] - before) / 10
         assert per_step <= 3 if fused else per_step > 3, per_step
+
+
+@pytest.mark.parametrize("name", ["walls_d3q15", "st_d3q15", "bubble_d3q15"])
+def test_table_candidate(gpu_lib, name):
+    """The neighbour-table kernels as a candidate of the fused D3Q15 path."""
+    from multiphaselb_b200 import Lattice
+    case = small_cases()[name]
+    k = orc.Checker("port", case)
+    k.upload_case()
+    k.initialize()
+    with Lattice(case, path=abi.PATH_FUSED, tile_config=6) as lat:
+        lat.upload_case()
+        lat.initialize()
+        for chunk in (1, 6):
+            k.step(chunk)
+            lat.step(chunk)
+            assert_same(lat.download(), k.download(), ctx=f"{name} after {chunk}")
+        assert lat.info()["tile_config"] == 5
