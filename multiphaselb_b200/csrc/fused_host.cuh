@@ -395,7 +395,10 @@ inline int node_programs(const Params& P, const std::vector<PatchDev>* fp, const
     progs.assign(1, BCProg{});
     any = false;
     {
-        std::vector<BCProg> node(n, BCProg{});
+        // programs of the patches' nodes only: an entry for every node of a large
+        // lattice would cost its page faults at each create
+        std::vector<uint32_t> slot(n, 0);
+        std::vector<BCProg> node(1, BCProg{});
         size_t off = 0;
         for (size_t p = 0; p < fp[0].size(); p++) {
             for (uint32_t i = 0; i < fp[0][p].count; i++) {
@@ -404,7 +407,11 @@ inline int node_programs(const Params& P, const std::vector<PatchDev>* fp, const
                     if (!(fi == 0 ? P.f_update : P.g_update)) continue;
                     int t = fp[fi][p].type;
                     if (t != MPLB_BC_BOUNCEBACK && t != MPLB_BC_FIXEDT) continue;
-                    BCProg& b = node[id];
+                    if (!slot[id]) {
+                        slot[id] = (uint32_t)node.size();
+                        node.push_back(BCProg{});
+                    }
+                    BCProg& b = node[slot[id]];
                     if (fi == 0) {
                         if (b.nf >= FUSED_MAX_OPS) { err = "too many boundary ops on one node"; return MPLB_E_UNSUPPORTED; }
                         b.ft[b.nf++] = (uint8_t)t;
@@ -419,8 +426,8 @@ inline int node_programs(const Params& P, const std::vector<PatchDev>* fp, const
             off += fp[0][p].count;
         }
         for (uint32_t id = 0; id < n; id++) {
-            const BCProg& b = node[id];
-            if (b.nf == 0 && b.ng == 0) continue;
+            if (!slot[id]) continue;
+            const BCProg& b = node[slot[id]];
             int found = -1;
             for (size_t q = 1; q < progs.size(); q++)
                 if (std::memcmp(&progs[q], &b, sizeof(BCProg)) == 0) { found = (int)q; break; }

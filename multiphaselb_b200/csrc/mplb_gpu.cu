@@ -96,6 +96,7 @@ struct mplb_gpu {
     int dev = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    cudaEvent_t table_done = nullptr;  // operator path on a caller's stream: after its last steps
     Params P{};
     int lat = 0, Q = 0, D = 0;
     uint32_t n = 0;
@@ -1023,6 +1024,7 @@ int table_enter(mplb_gpu* h) {
         h->T2 = buf[1];
         h->U2 = buf[2];
     }
+    if (!h->own_stream && !h->table_done) CK(cudaEventCreateWithFlags(&h->table_done, cudaEventDisableTiming));
     if (h->fstate == 0) {
         RET(DISPATCH(h, op_collision, h, 0));
         RET(DISPATCH(h, op_collision, h, 1));
@@ -1040,7 +1042,40 @@ struct NodeCopy {
 int copy_node_rows(mplb_gpu* dst, uint32_t dst_start, mplb_gpu* src, uint32_t src_start, uint32_t count,
                    const NodeCopy* parts, int np);
 
+// A caller that captures its stream into a graph may replay the graph from any
+// later state of the handle, which the table kernels, whose state between
+// steps is not the reference's, could not serve.  At the first capture the
+// handle goes back to the operators for good; the state of the steps before is
+// rebuilt at once, on a stream of its own and outside the graph.
+int table_leave_if_capturing(mplb_gpu* h) {
+    if (!h->table || h->own_stream) return 0;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) cudaGetLastError();
+    if (st == cudaStreamCaptureStatusNone) return 0;
+    if (h->fstate != 0) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        CK(cudaThreadExchangeStreamCaptureMode(&mode));
+        cudaStream_t side = nullptr, own = h->stream;
+        int rc = 0;
+        if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) rc = fail(MPLB_E_CUDA, "stream");
+        if (!rc && cudaStreamWaitEvent(side, h->table_done, 0) != cudaSuccess) rc = fail(MPLB_E_CUDA, "event");
+        if (!rc) {
+            h->stream = side;
+            rc = table_step(h, true);
+            h->stream = own;
+        }
+        if (side && cudaStreamSynchronize(side) != cudaSuccess && !rc) rc = fail(MPLB_E_CUDA, "table state");
+        if (side) cudaStreamDestroy(side);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (rc) return rc;
+        h->fstate = 0;
+    }
+    h->table = false;
+    return 0;
+}
+
 int materialize(mplb_gpu* h) {
+    RET(table_leave_if_capturing(h));
     if (h->fstate == 0) return 0;
     if (h->path == MPLB_PATH_OPERATORS) RET(table_step(h, true));
     else if (h->precision == MPLB_FP32_DEV) RET(fused32_step(h, true));
@@ -1349,6 +1384,7 @@ int mplb_gpu_destroy(mplb_gpu_t* h) {
         cudaStreamDestroy(h->snap_stream);
     }
     if (h->order_ev) cudaEventDestroy(h->order_ev);
+    if (h->table_done) cudaEventDestroy(h->table_done);
     if (h->snap_ready) cudaEventDestroy(h->snap_ready);
     if (h->snap_done) cudaEventDestroy(h->snap_done);
     if (h->snap_dev) cudaFree(h->snap_dev);
@@ -1443,9 +1479,11 @@ int mplb_gpu_step(mplb_gpu_t* h, uint32_t nsteps) {
         h->current += nsteps;
         return 0;
     }
+    RET(table_leave_if_capturing(h));
     if (h->table) RET(table_enter(h));
     if (h->table) {
         for (uint32_t s = 0; s < nsteps; s++) RET(table_step(h, false));
+        if (h->table_done) CK(cudaEventRecord(h->table_done, h->stream));
         h->current += nsteps;
         return 0;
     }

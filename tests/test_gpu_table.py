@@ -77,3 +77,37 @@ def test_table_candidate(gpu_lib, name):
             lat.step(chunk)
             assert_same(lat.download(), k.download(), ctx=f"{name} after {chunk}")
         assert lat.info()["tile_config"] == 5
+
+
+@pytest.mark.parametrize("warmup", [0, 3])
+@pytest.mark.parametrize("name", ["cylinder_d2q9", "my_column_d2q9", "bubble_d2q9"])
+def test_captured_steps(gpu_lib, name, warmup):
+    """Steps captured on the caller's stream replay as the operators do: from
+    the state the handle holds then, also after downloads and other steps."""
+    import torch
+
+    from multiphaselb_b200 import Lattice
+    case = small_cases()[name]
+    k = orc.Checker("port", case)
+    k.upload_case()
+    k.initialize()
+    stream = torch.cuda.Stream()
+    with Lattice(case, path=abi.PATH_OPERATORS, stream=stream.cuda_stream) as lat:
+        lat.upload_case()
+        lat.initialize()
+        if warmup:
+            lat.step(warmup)
+            k.step(warmup)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            lat.step(2)
+        for replays in (1, 2):
+            for _ in range(replays):
+                with torch.cuda.stream(stream):
+                    graph.replay()
+                k.step(2)
+            assert_same(lat.download(), k.download(), ctx=f"{name} after {replays} replays")
+            lat.step(2)
+            k.step(2)
+        del graph
