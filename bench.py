@@ -261,12 +261,20 @@ def measure(case, path, precision, steps, warmup, local, stream, flush, world, d
 
 
 def kernel_name(case, precision, tile_config=-1):
-    """The step kernel the autotuner picked (3D candidates 6 to 9 are the TMA-staged kernel)."""
+    """The step kernel in use.  FP64: the autotuner's pick (2D candidate 10 is
+    the myMRT march, 3D candidate 5 the neighbour-table kernels, 6 to 9 the
+    TMA-staged kernel).  FP32 in 3D: a box without boundary patches whose x
+    and y extents are multiples of 32 and 8 takes the TMA-staged kernel."""
     from multiphaselb_b200 import abi
     if precision == abi.FP32_DEV:
-        return "k_fused32_d2q9" if case.lattice == abi.D2Q9 else "k_fused32_d3q15"
+        if case.lattice == abi.D2Q9:
+            return "k_fused32_d2q9"
+        nx, ny = case.dims[0], case.dims[1]
+        return "k_fused32_d3q15_tma" if not case.patches and nx % 32 == 0 and ny % 8 == 0 else "k_fused32_d3q15"
     if case.lattice == abi.D2Q9:
-        return "k_fused_d2q9"
+        return "k_march_my_d2q9" if tile_config == 10 else "k_fused_d2q9"
+    if tile_config == 5:
+        return "k_table_sum + k_table_finish"
     return "k_fused_d3q15_tma" if tile_config in (6, 7, 8, 9) else "k_fused_d3q15"
 
 

@@ -75,7 +75,8 @@ enum { MPLB_FP64 = 0, MPLB_FP32_DEV = 1 };
 /* Execution path. */
 enum {
     MPLB_PATH_AUTO = 0,      /* fused box kernels when the mesh is a box, else operators */
-    MPLB_PATH_OPERATORS = 1, /* one kernel per reference operator, neighbour-table driven */
+    MPLB_PATH_OPERATORS = 1, /* neighbour-table driven: the reference's operators one by one; a
+                                whole step in two or three kernels where every boundary allows */
     MPLB_PATH_FUSED = 2      /* fused box kernels; create fails if the mesh is not a box */
 };
 
