@@ -235,6 +235,10 @@ __global__ void __launch_bounds__(TX * TY, MINB)
         mul_M<L, 1>(fp, m);
         // one decision for the whole block: a wait that ran out in any thread ends the kernel
         if (!mbar_wait_bounded(psi_bar, (uint32_t)j & 1u, TMA_WAIT_LIMIT) || *s_fail) {
+            *s_fail = 1;
+            if (face)
+                leave_face_tile(j, G::NSTAGE, fparity, p + 1 <= plast, [&](int t) { mbar_arrive(&face_bar[t]); },
+                                [&](int t, uint32_t par) { mbar_wait_bounded(&face_bar[t], par, TMA_WAIT_LIMIT); });
             failed = true;
             break;
         }
@@ -268,6 +272,7 @@ __global__ void __launch_bounds__(TX * TY, MINB)
     if (failed) {
         if (tid == 0) atomicExch(A.kerr, MPLB_KERR_WAIT);
         // let the copies this block issued land before its shared memory is released
+        // (the bulk copies of wrapped parts: leave_face_tile)
         cp_async_wait_all();
         for (int s = 0; s < G::NSTAGE; s++)
             if ((pending >> s) & 1u) mbar_wait_bounded(&bar[s], (parity >> s) & 1u, TMA_WAIT_LIMIT);

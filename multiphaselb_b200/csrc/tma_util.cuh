@@ -87,6 +87,20 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// A thread of a face tile gives up at plane step j, a wait of its block having
+// run out; fparity: per stage, the parity of its next wait for wrapped parts
+// (that of stage j % nstage toggled already).  It takes no part in writing the
+// wrapped parts of the next plane, so it arrives for them (more: there is one):
+// threads that have written theirs can still see the phase complete.  Then it
+// waits for the parts of plane j, the last whose bulk copies it may have in
+// flight: shared memory must not be released under them.  wait() is bounded.
+template <class Arrive, class Wait>
+MPLB_HD void leave_face_tile(int j, int nstage, uint32_t fparity, bool more, Arrive arrive, Wait wait) {
+    const int s = j % nstage;
+    if (more) arrive((j + 1) % nstage);
+    wait(s, ((fparity >> s) & 1u) ^ 1u);
+}
+
 // c within one extent of [0, ext): wrapped into it
 MPLB_HD int wrap_any(int c, int ext) { return c < 0 ? c + ext : (c >= ext ? c - ext : c); }
 
