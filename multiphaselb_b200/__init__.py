@@ -152,6 +152,7 @@ class Lattice:
                                               C.byref(self._desc.f), C.byref(self._desc.g),
                                               C.byref(opts), C.byref(h)))
         self.h = h
+        self._batches = []  # handles of the batches that hold this lattice
 
     # ---------------------------------------------------------------- plumbing
     def _check(self, rc):
@@ -160,6 +161,8 @@ class Lattice:
 
     def close(self):
         if getattr(self, "h", None):
+            for b in self._batches:
+                b.close()
             self.lib.mplb_gpu_destroy(self.h)
             self.h = None
 
@@ -334,12 +337,27 @@ class Lattice:
         return m.value, e.value
 
 
+class _BatchHandle:
+    """A C-ABI batch, destroyed once: by its Batch, or by the first of its
+    lattices that closes.  The lattices must outlive it, and Python's own order
+    cannot be relied on (objects of a cycle, a script's globals at exit); the
+    lattices hold this object, not the Batch, which they would keep alive."""
+
+    def __init__(self, lib, h):
+        self.lib, self.h = lib, h
+
+    def close(self):
+        if self.h:
+            self.lib.mplb_batch_destroy(self.h)
+            self.h = None
+
+
 class Batch:
     """Many independent lattices advanced together (mplb_batch_*).
 
     ``lattices`` are :class:`Lattice` objects (D2Q9, FP32-deviation, fused,
-    fully periodic, isothermal); they stay usable between batch calls and
-    must outlive the batch.
+    fully periodic, isothermal); they stay usable between batch calls.
+    Closing one of them closes the batch.
     """
 
     def __init__(self, lattices, check_interval=1000, tol=1e-9, tile_config=0):
@@ -349,16 +367,21 @@ class Batch:
         opts = abi.BatchOpts(tile_config, check_interval, tol)
         h = C.c_void_p()
         self._check(self.lib.mplb_batch_create(arr, len(self.lattices), C.byref(opts), C.byref(h)))
-        self.h = h
+        self._handle = _BatchHandle(self.lib, h)
+        for lat in self.lattices:
+            lat._batches = [b for b in lat._batches if b.h] + [self._handle]
+
+    @property
+    def h(self):
+        return self._handle.h
 
     def _check(self, rc):
         if rc != 0:
             raise MplbError(rc, self.lib.mplb_gpu_last_error().decode())
 
     def close(self):
-        if getattr(self, "h", None):
-            self.lib.mplb_batch_destroy(self.h)
-            self.h = None
+        if getattr(self, "_handle", None):
+            self._handle.close()
 
     def __del__(self):
         try:
