@@ -1000,6 +1000,15 @@ int table_step(mplb_gpu* h, bool emit) {
     return 0;
 }
 
+// While this lives, the calling thread may allocate and wait although some other
+// stream is being captured (a step of this handle is no part of that capture,
+// and the operators, which the table kernels stand for, allocate nothing).
+struct AnyCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Enter the fused state.  Without memory for the kernels' buffers the lattice
 // stays on the operators.
 int table_enter(mplb_gpu* h) {
@@ -1007,10 +1016,16 @@ int table_enter(mplb_gpu* h) {
         const bool gon = h->P.g_update != 0;
         double* buf[3] = {nullptr, nullptr, nullptr};
         const size_t count[3] = {2 * (size_t)h->n, gon ? (size_t)h->n : 0, gon ? 3 * (size_t)h->n : 0};
-        for (int i = 0; i < 3; i++) {
-            if (!count[i] || cudaMalloc((void**)&buf[i], count[i] * sizeof(double)) == cudaSuccess) continue;
+        bool got = true;
+        {
+            AnyCapture guard;
+            for (int i = 0; i < 3 && got; i++)
+                got = !count[i] || cudaMalloc((void**)&buf[i], count[i] * sizeof(double)) == cudaSuccess;
+            if (!got)
+                for (double* b : buf) cudaFree(b);
+        }
+        if (!got) {
             cudaGetLastError();
-            for (double* b : buf) cudaFree(b);
             h->table = false;
             return 0;
         }
@@ -1053,8 +1068,7 @@ int table_leave_if_capturing(mplb_gpu* h) {
     if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) cudaGetLastError();
     if (st == cudaStreamCaptureStatusNone) return 0;
     if (h->fstate != 0) {
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        CK(cudaThreadExchangeStreamCaptureMode(&mode));
+        AnyCapture guard;
         cudaStream_t side = nullptr, own = h->stream;
         int rc = 0;
         if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) rc = fail(MPLB_E_CUDA, "stream");
@@ -1066,7 +1080,6 @@ int table_leave_if_capturing(mplb_gpu* h) {
         }
         if (side && cudaStreamSynchronize(side) != cudaSuccess && !rc) rc = fail(MPLB_E_CUDA, "table state");
         if (side) cudaStreamDestroy(side);
-        cudaThreadExchangeStreamCaptureMode(&mode);
         if (rc) return rc;
         h->fstate = 0;
     }
