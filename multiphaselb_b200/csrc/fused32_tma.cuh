@@ -15,6 +15,7 @@
 #pragma once
 
 #include "fused32.cuh"
+#include "tma_maps.h"
 #include "tma_util.cuh"
 
 namespace mplb {
@@ -35,6 +36,27 @@ struct TmaTile32 {
 // Candidate box: what the kernel takes.
 inline bool tma3_fits32(int nx, int ny, int nz, int px, int py, int pz, bool has_bc, int TX, int TY) {
     return !has_bc && px && py && pz && nx % TX == 0 && ny % TY == 0 && nz >= 2;
+}
+
+// The TMA-staged kernel's tile for a box, and its tensor maps of the step's input
+// buffers.  64 x 8 where it divides the box, else 32 x 8 at two blocks per SM
+// (more halo per node): us per step on 192^3 338 and 357 against 438 of the
+// general kernel, on 64^3 22.4 and 22.5 against 27.3 (B200).  tile -1: the
+// general kernel steps this lattice (the box, or no maps to be had).
+struct Tma32 {
+    int tile = -1;  // 0: 64 x 8, 1: 32 x 8
+    const TmaMaps* maps = nullptr;
+};
+inline Tma32 tma32_choose(TmaMapCache& cache, PFN_cuTensorMapEncodeTiled_v12000 enc, const FusedArgs& A, bool has_bc,
+                          uint32_t n, const float* fin, const double* Told) {
+    Tma32 r;
+    if (tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 64, 8)) r.tile = 0;
+    else if (tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 32, 8)) r.tile = 1;
+    else return r;
+    const int tx = r.tile == 0 ? 64 : 32, ty = 8;
+    r.maps = cache.get(enc, r.tile, A.nx, A.ny, A.nz, fin, true, Told, n, tx + 8, ty + 2, tx + 4);
+    if (!r.maps) r.tile = -1;
+    return r;
 }
 
 template <int TX, int TY, int MINB>

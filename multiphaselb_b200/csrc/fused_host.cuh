@@ -4,12 +4,11 @@
 // object (compiled without multiply-add contraction).
 #pragma once
 
-#include <cudaTypedefs.h>
-
 #include "fused.cuh"
 #include "fused_march.cuh"
 #include "fused_table.cuh"
 #include "fused_tma.cuh"
+#include "tma_maps.h"
 
 // The marching D2Q9 step with myMRT heat (mplb_march.cu).
 int mplb_march_resident(bool f_on, bool bc);
@@ -20,16 +19,6 @@ int mplb_table_step(int lat, int heat, bool emit, bool st, const mplb::Params& P
                     cudaStream_t s);
 
 namespace mplb {
-
-// Tensor maps of one TMA candidate over one input population buffer and the
-// temperature field (a map holds its box shape, so each candidate has its own).
-struct TmaMaps {
-    int cfg = -1;
-    const void* f = nullptr;
-    const void* T = nullptr;
-    alignas(64) CUtensorMap mf;
-    alignas(64) CUtensorMap mT;
-};
 
 struct FusedConfig {
     std::string err;
@@ -50,61 +39,8 @@ struct FusedConfig {
     int tile_cfg = 2;
     int* kerr = nullptr;           // kernel error flag (bounded waits), one int
     int* kerr_host = nullptr;      // its pinned host copy
-    TmaMaps tmaps[4];              // two TMA candidates x two population buffers
-    int tmaps_next = 0;
+    TmaMapCache tmaps;
 };
-
-// cuTensorMapEncodeTiled from the driver, found through the runtime (the
-// library does not link the driver API).
-inline PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }();
-    return fn;
-}
-
-// Tensor maps of a step's input buffers: the populations (FP64 or FP32) as a
-// 4D tensor (x, y, z, k) with boxes of bx x by, T as a 3D one (x, y, z) with
-// boxes of tbx x by; no swizzle, zero fill (never read: the kernels take
-// tensor copies only for boxes inside the lattice).  Kept per (key, buffers).
-inline const TmaMaps* tma_maps(FusedConfig& fc, int key, const FusedArgs& A, const void* fin, bool fp32,
-                               const double* Told, uint32_t n, int bx, int by, int tbx) {
-    for (const TmaMaps& m : fc.tmaps)
-        if (m.cfg == key && m.f == fin && m.T == Told) return &m;
-    auto enc = tensor_map_encoder();
-    if (!enc) {
-        fc.err = "cuTensorMapEncodeTiled is not available from the driver";
-        return nullptr;
-    }
-    TmaMaps& m = fc.tmaps[fc.tmaps_next];
-    const cuuint64_t dims[4] = {(cuuint64_t)A.nx, (cuuint64_t)A.ny, (cuuint64_t)A.nz, 15};
-    auto encode = [&](CUtensorMap* map, bool f32, int rank, const void* p, int width) {
-        const cuuint64_t es = f32 ? 4 : 8;
-        const cuuint64_t strides[3] = {(cuuint64_t)A.nx * es, (cuuint64_t)A.nx * A.ny * es, (cuuint64_t)n * es};
-        const cuuint32_t box[4] = {(cuuint32_t)width, (cuuint32_t)by, 1, 1};
-        const cuuint32_t step[4] = {1, 1, 1, 1};
-        return enc(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, rank,
-                   const_cast<void*>(p), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    };
-    CUresult r = encode(&m.mf, fp32, 4, fin, bx);
-    if (r == CUDA_SUCCESS) r = encode(&m.mT, false, 3, Told, tbx);
-    if (r != CUDA_SUCCESS) {
-        fc.err = "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")";
-        m.cfg = -1;
-        return nullptr;
-    }
-    m.cfg = key;
-    m.f = fin;
-    m.T = Told;
-    fc.tmaps_next = (fc.tmaps_next + 1) % 4;
-    return &m;
-}
 
 template <int TX, int TY, bool PIPE, bool HAS_BC, bool EMIT, bool ST = false>
 cudaError_t set_smem3() {
@@ -146,7 +82,8 @@ inline cudaError_t fused_attributes() {
 
 template <int TX, int TY, int MINB>
 cudaError_t launch3_tma(FusedConfig& fc, int cfg, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
-    const TmaMaps* m = tma_maps(fc, cfg, A, A.fin, false, A.Told, P.n, TX + 4, TY + 2, TX + 4);
+    const TmaMaps* m = fc.tmaps.get(tensor_map_encoder(), cfg, A.nx, A.ny, A.nz, A.fin, false, A.Told, P.n, TX + 4, TY + 2,
+                                    TX + 4);
     if (!m) return cudaErrorInvalidValue;
     if (P.st_on) launch_step(k_fused_d3q15_tma<TX, TY, MINB, true>, nb, TX * TY, TmaTile<TX, TY>::SMEM, s, P, A, m->mf, m->mT);
     else launch_step(k_fused_d3q15_tma<TX, TY, MINB>, nb, TX * TY, TmaTile<TX, TY>::SMEM, s, P, A, m->mf, m->mT);

@@ -305,19 +305,7 @@ FusedArgs32 mplb_make_args32(const FusedArgs& A, const Params& P, double rho_ref
     return B;
 }
 
-// TMA-staged 3D step: the tile for this box (-1: the general kernel takes it),
-// its extents for the tensor maps, and a launch.  64 x 8 where it divides the
-// box, else 32 x 8 at two blocks per SM (more halo per node): us per step on
-// 192^3 338 and 357 against 438 of the general kernel, on 64^3 22.4 and 22.5
-// against 27.3 (B200).
-int mplb_tma32_pick(const FusedArgs& A, bool has_bc) {
-    if (tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 64, 8)) return 0;
-    return tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 32, 8) ? 1 : -1;
-}
-void mplb_tma32_tile(int c, int* tx, int* ty) {
-    *tx = c == 0 ? 64 : 32;
-    *ty = 8;
-}
+// A launch of the TMA-staged 3D step (c: Tma32::tile).
 cudaError_t mplb_tma32_launch(int c, FusedArgs32 B, const Params& P, const CUtensorMap& mf, const CUtensorMap& mT,
                               cudaStream_t s) {
     FusedArgs tmp{};

@@ -20,7 +20,7 @@
 #include "mplb_io.h"
 #include "ops.cuh"
 #include "fused_host.cuh"
-#include "fused32.cuh"
+#include "fused32_tma.cuh"
 #include "fused_table.cuh"
 
 using namespace mplb;
@@ -32,8 +32,6 @@ int mplb_fused32_attributes();
 cudaError_t mplb_fused32_launch(int lat, bool has_bc, bool f_on, bool g_on, bool emit, FusedArgs32 B, const Params& P,
                                 double* emit_f, double* emit_g, double* rho_out, double* Fi_out, double* Ft_out,
                                 cudaStream_t s);
-int mplb_tma32_pick(const FusedArgs& A, bool has_bc);
-void mplb_tma32_tile(int c, int* tx, int* ty);
 cudaError_t mplb_tma32_launch(int c, FusedArgs32 B, const Params& P, const CUtensorMap& mf, const CUtensorMap& mT,
                               cudaStream_t s);
 cudaError_t mplb_to_dev32(uint32_t n, int Q, const double* src, float* dst, const FusedArgs32& B, int heat,
@@ -874,14 +872,12 @@ int fused32_step(mplb_gpu* h, bool emit) {
     B.Unew = udb ? (emit ? h->U : h->U2) : h->U;
     B.S = h->S;
     B.rho_c = h->rho;
-    const int tma = !emit && h->lat == MPLB_D3Q15 ? mplb_tma32_pick(h->fc.args, h->fc.has_bc) : -1;
+    Tma32 tma;
+    if (!emit && h->lat == MPLB_D3Q15)
+        tma = tma32_choose(h->fc.tmaps, tensor_map_encoder(), h->fc.args, h->fc.has_bc, h->n, B.fin, B.Told);
     cudaError_t e;
-    if (tma >= 0) {
-        int tx, ty;
-        mplb_tma32_tile(tma, &tx, &ty);
-        const TmaMaps* m = tma_maps(h->fc, tma, h->fc.args, B.fin, true, B.Told, h->n, tx + 8, ty + 2, tx + 4);
-        if (!m) return fail(MPLB_E_CUDA, h->fc.err);
-        e = mplb_tma32_launch(tma, B, h->P, m->mf, m->mT, h->stream);
+    if (tma.tile >= 0) {
+        e = mplb_tma32_launch(tma.tile, B, h->P, tma.maps->mf, tma.maps->mT, h->stream);
     } else {
         e = mplb_fused32_launch(h->lat, h->fc.has_bc, fon, gon, emit, B, h->P, fon ? h->F() : nullptr,
                                 gon ? h->G() : nullptr, h->rho, h->Fi, h->Ft, h->stream);
