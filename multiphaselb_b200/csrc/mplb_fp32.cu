@@ -180,11 +180,9 @@ constexpr size_t f3_smem32() {
     return (size_t)3 * (TY + 2) * (TX + 2) * sizeof(double) + (size_t)2 * 15 * TX * TY * sizeof(float);
 }
 
-// The step's 32 x 4 tiles ask for five blocks per SM (at most 96 registers):
-// 101 x 75 x 90 periodic 52 us a step against 66 with four blocks of the 122
-// registers that the allocator takes otherwise (B200).
-template <int TX, int TY, bool HAS_BC, bool EMIT>
-__global__ void __launch_bounds__(TX * TY, !EMIT && TX * TY == 128 ? 5 : min_blocks(TX * TY))
+// MINB: blocks per SM asked of the register allocator (0: min_blocks).
+template <int TX, int TY, bool HAS_BC, bool EMIT, int MINB = 0>
+__global__ void __launch_bounds__(TX * TY, MINB ? MINB : min_blocks(TX * TY))
     k_fused32_d3q15(Params P, FusedArgs32 A, double* emit_f, double* rho_out, double* Fi_out, double* Ft_out) {
     step_dependency_wait();
     using L = D3Q15T;
@@ -263,9 +261,9 @@ __global__ void __launch_bounds__(TX * TY, !EMIT && TX * TY == 128 ? 5 : min_blo
     }
 }
 
-template <int TX, int TY, bool BC, bool EMIT>
+template <int TX, int TY, bool BC, bool EMIT, int MINB = 0>
 static cudaError_t set32() {
-    return cudaFuncSetAttribute(k_fused32_d3q15<TX, TY, BC, EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_fused32_d3q15<TX, TY, BC, EMIT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)f3_smem32<TX, TY>());
 }
 
@@ -326,8 +324,9 @@ int mplb_fused32_attributes() {
                              (int)TmaTile32<32, 8>::SMEM));
     chk(set32<32, 8, true, true>());
     chk(set32<32, 8, false, true>());
-    chk(set32<32, 4, true, false>());
-    chk(set32<32, 4, false, false>());
+    chk(set32<32, 4, true, false, 5>());
+    chk(set32<32, 4, false, false, 4>());
+    chk(set32<32, 4, false, false, 5>());
     return e == cudaSuccess ? 0 : -1;
 }
 
@@ -367,8 +366,12 @@ cudaError_t mplb_fused32_launch(int lat, bool has_bc, bool f_on, bool g_on, bool
         } else {
             const Geom g = fused_geometry(MPLB_D3Q15, tmp, 32, 4);
             B.tiles_x = g.tiles_x; B.tiles_y = g.tiles_y; B.zchunk = g.zchunk;
-            if (has_bc) launch_step(k_fused32_d3q15<32, 4, true, false>, g.nblocks, 128, f3_smem32<32, 4>(), s, P, B, emit_f, rho_out, Fi_out, Ft_out);
-            else launch_step(k_fused32_d3q15<32, 4, false, false>, g.nblocks, 128, f3_smem32<32, 4>(), s, P, B, emit_f, rho_out, Fi_out, Ft_out);
+            auto go = [&](auto kern) {
+                launch_step(kern, g.nblocks, 128, f3_smem32<32, 4>(), s, P, B, emit_f, rho_out, Fi_out, Ft_out);
+            };
+            if (has_bc) go(k_fused32_d3q15<32, 4, true, false, 5>);
+            else if (general32_blocks(g, B.nz) == 4) go(k_fused32_d3q15<32, 4, false, false, 4>);
+            else go(k_fused32_d3q15<32, 4, false, false, 5>);
         }
     }
     return cudaGetLastError();
