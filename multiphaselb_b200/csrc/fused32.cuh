@@ -624,16 +624,16 @@ __device__ __forceinline__ void finish_node32(const Params& P, const FusedArgs32
 
 // Blocks per SM that the general 3D step without boundary programs asks for, its
 // launch being g (32 x 4 tiles): five (96 registers) or four (122).  Five hold
-// more of a large lattice at once, but where all blocks fit at four per SM (592;
-// the short chunks at the top may wait), five put a fifth on some SMs, which
-// then set the time.  B200, us per step at four and five: 304 blocks 33 and 29,
-// 420 blocks 39.1 and 34.6, 464 blocks 39.9 and 52.2, 584 blocks 40.4 and 53.3,
-// 320 full and 320 short ones 39.9 and 52.3, 600 blocks 34.4 and 30.1, 912 blocks
-// 66.7 and 52.7; up to 296 blocks within 2 %.  With boundary programs both take
-// 96 registers or less and the same time.
+// more of a large lattice at once, but where all blocks fit at four per SM (592,
+// or a few short chunks of the top planes more), five put a fifth on some SMs,
+// which then set the time.  B200, us per step at four and five: 304 blocks 33 and
+// 29, 420 blocks 39.1 and 34.6, 464 blocks 39.9 and 52.2, 584 blocks 40.4 and
+// 53.3, 320 full and 320 short ones 39.9 and 52.3, 512 and 512 63.3 and 56.5, 600
+// full ones 34.4 and 30.1, 912 66.7 and 52.7; up to 296 blocks within 2 %.  With
+// boundary programs both take 96 registers or less and the same time.
 inline int general32_blocks(const Geom& g, int nz) {
     const int full = g.tiles_x * g.tiles_y * (nz / g.zchunk);  // blocks of whole chunks
-    return g.nblocks > 3 * 148 && full <= 4 * 148 ? 4 : 5;
+    return g.nblocks > 3 * 148 && full <= 4 * 148 && g.nblocks <= 4 * 148 + 74 ? 4 : 5;
 }
 
 }  // namespace mplb

@@ -38,11 +38,48 @@ inline bool tma3_fits32(int nx, int ny, int nz, int px, int py, int pz, bool has
     return !has_bc && px && py && pz && nx % TX == 0 && ny % TY == 0 && nz >= 2;
 }
 
-// The TMA-staged kernel's tile for a box, and its tensor maps of the step's input
-// buffers.  64 x 8 where it divides the box, else 32 x 8 at two blocks per SM
-// (more halo per node): us per step on 192^3 338 and 357 against 438 of the
-// general kernel, on 64^3 22.4 and 22.5 against 27.3 (B200).  tile -1: the
-// general kernel steps this lattice (the box, or no maps to be had).
+// The kernel that steps a box without boundary programs: 0, 1 the TMA-staged one
+// with 64 x 8 tiles (one block per SM) or 32 x 8 (two, more halo per node), -1
+// the general one.  By an estimate of its time, in us on a B200: rounds of
+// resident blocks, times the planes of a block, times what a plane took.  The
+// TMA kernel's plane is the longer one: 3.5 us; with 32 x 8 tiles 2.8, two per
+// SM 3.6; a fifth more where a tile's rows lie on both y faces; general 2.25,
+// 2.75, 3.25 and 3.95 with one to four blocks per SM, 5.5 with five.  Its chunks
+// may be shorter, though, four planes instead of eight, to fill the device.
+// (The planes beside a chunk count in full but for the general kernel at four
+// and more blocks per SM, and a round that is not full costs that kernel half of
+// one, unless nearly empty.)  So flat boxes and slabs of a few planes take the
+// general kernel and large boxes the TMA one.  Measured, us per step, general,
+// 64 x 8, 32 x 8: 64 x 8 x 4 13.8, 24.7, 21.2; 64 x 64 x 4 14.0, 21.9, 18.1;
+// 320 x 320 x 2 18.9, 28.6, 25.1; 512 x 512 x 2 46.6, 55.4, 50.1; 64 x 64 x 16
+// 24.5, 22.3, 18.3; 192 x 192 x 8 28.7, 23.6, 24.0; 512 x 512 x 16 250, 252, 242;
+// 128^3 126, 121, 127; 192^3 438, 338, 357.
+inline int tma32_tile(const FusedArgs& A, bool has_bc) {
+    if (!tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 32, 8)) return -1;
+    const double edge = A.ny == 8 ? 1.2 : 1.0;
+    const Geom g = fused_geometry(MPLB_D3Q15, A, 32, 4);
+    const double per_sm = g.nblocks / 148.0;
+    const double rounds = (double)g.tiles_x * g.tiles_y * A.nz / g.zchunk / (5 * 148);
+    double best = general32_blocks(g, A.nz) == 4 ? (g.zchunk + 1.6) * 3.95
+                  : per_sm <= 4 ? (g.zchunk + 2) * (per_sm <= 1 ? 2.25 : per_sm <= 2 ? 2.75 : 3.25)
+                                : (g.zchunk + 1.3) * 5.5 * (rounds <= 1.2 ? std::max(1.0, rounds) : std::max(1.5, rounds));
+    int pick = -1;
+    if (A.nx % 64 == 0) {
+        const Geom t = resident_geometry(A, 64, 8, 1);
+        const double us = 1.2 + (t.zchunk + 2) * edge * 3.5 * ((t.nblocks + 147) / 148);
+        if (us < best) {
+            best = us;
+            pick = 0;
+        }
+    }
+    const Geom t = resident_geometry(A, 32, 8, 2);
+    const int rest = t.nblocks % 296;
+    const double us = 1.2 + (t.zchunk + 2) * edge * (3.6 * (t.nblocks / 296) + (rest == 0 ? 0.0 : rest <= 148 ? 2.8 : 3.6));
+    return us < best ? 1 : pick;
+}
+
+// That kernel and, for the TMA-staged one, the tensor maps of the step's input
+// buffers.  tile -1: the general kernel (the box, or no maps to be had).
 struct Tma32 {
     int tile = -1;  // 0: 64 x 8, 1: 32 x 8
     const TmaMaps* maps = nullptr;
@@ -50,9 +87,8 @@ struct Tma32 {
 inline Tma32 tma32_choose(TmaMapCache& cache, PFN_cuTensorMapEncodeTiled_v12000 enc, const FusedArgs& A, bool has_bc,
                           uint32_t n, const float* fin, const double* Told) {
     Tma32 r;
-    if (tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 64, 8)) r.tile = 0;
-    else if (tma3_fits32(A.nx, A.ny, A.nz, A.px, A.py, A.pz, has_bc, 32, 8)) r.tile = 1;
-    else return r;
+    r.tile = tma32_tile(A, has_bc);
+    if (r.tile < 0) return r;
     const int tx = r.tile == 0 ? 64 : 32, ty = 8;
     r.maps = cache.get(enc, r.tile, A.nx, A.ny, A.nz, fin, true, Told, n, tx + 8, ty + 2, tx + 4);
     if (!r.maps) r.tile = -1;

@@ -28,10 +28,13 @@ def test_rule_on_the_host():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dims", [(250, 250, 2), (60, 58, 128)])
-def test_general_kernel_at_four_blocks_per_sm(gpu_lib, dims):
-    """504 and 480 blocks of 32 x 4 tiles, partial ones among them; the bounds
-    are those of six FP32 steps at other sizes (test_tma_staging.py)."""
+@pytest.mark.parametrize("dims", [(250, 250, 2), (60, 58, 128), (64, 64, 4), (320, 256, 2), (64, 8, 8), (64, 16, 9),
+                                  (192, 192, 8), (128, 128, 64)])
+def test_kernels_match_oracle(gpu_lib, dims):
+    """The general kernel at four blocks per SM (504 and 480 blocks, partial tiles
+    among them) and on flat boxes that the TMA tiles divide, and the TMA-staged
+    kernel with either tile; the bounds are those of six FP32 steps at other
+    sizes (test_tma_staging.py)."""
     from multiphaselb_b200 import Lattice
     case = cases.perturbed(cases.bubble_case(abi.D3Q15, 8, 2.5, 3.0, 0.75, dims=dims), du=1e-3)
     want = run_checker("port", case, 6)
