@@ -21,11 +21,12 @@ LIB = os.path.join(LIB_DIR, "libmplb_gpu.so")
 SOURCES = [(os.path.join(HERE, "csrc", "mplb_gpu.cu"), False),
            (os.path.join(HERE, "csrc", "mplb_march.cu"), False),
            (os.path.join(HERE, "csrc", "mplb_table.cu"), False),
+           (os.path.join(HERE, "csrc", "mplb_st.cu"), False),
            (os.path.join(HERE, "csrc", "mplb_noalloc.cu"), False),
            (os.path.join(HERE, "csrc", "mplb_fp32.cu"), True),
            (os.path.join(HERE, "csrc", "mplb_mlp.cu"), False),
            (os.path.join(HERE, "csrc", "mplb_io.cu"), False)]
-HEADERS = [os.path.join(HERE, "csrc", f) for f in ("lattice.cuh", "ops.cuh", "fused.cuh", "fused_host.cuh", "fused_march.cuh", "fused_table.cuh", "fused_tma.cuh", "tma_util.cuh", "tma_maps.h", "umma.cuh", "fused32.cuh", "fused32_tma.cuh", "mplb_io.h")] + \
+HEADERS = [os.path.join(HERE, "csrc", f) for f in ("lattice.cuh", "ops.cuh", "fused.cuh", "fused_host.cuh", "fused_launch.cuh", "fused_march.cuh", "fused_table.cuh", "fused_tma.cuh", "tma_util.cuh", "tma_maps.h", "umma.cuh", "fused32.cuh", "fused32_tma.cuh", "mplb_io.h")] + \
           [os.path.join(ROOT, "include", "mplb_gpu.h")]
 
 NVCC_FLAGS = [

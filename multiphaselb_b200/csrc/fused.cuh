@@ -405,15 +405,22 @@ __device__ __forceinline__ void finish_node(const Params& P, const FusedArgs& A,
         return;
     }
     if constexpr (F_ON) {
-        // surface-tension term (zero on wall nodes, which miss a neighbour)
+        // surface-tension term (zero on wall nodes, which miss a neighbour).  Before
+        // the collision, not where it is added: the capped kernels spill less
+        // (2048^2 174 us a step against 183, one-wave lattices within 3 %; B200).
+        double C[ST ? L::Q : 1];
+        if constexpr (ST) {
+            if (!onb) {
+                surface_tension<L>(P, psi, nbpsi, C);
+            } else {
+#pragma unroll
+                for (int k = 0; k < L::Q; k++) C[k] = 0;
+            }
+        }
         auto term = [&](double* m) {
             if constexpr (ST) {
-                if (!onb) {
-                    double C[L::Q];
-                    surface_tension<L>(P, psi, nbpsi, C);
 #pragma unroll
-                    for (int k = 0; k < L::Q; k++) m[k] = m[k] + C[k];
-                }
+                for (int k = 0; k < L::Q; k++) m[k] = m[k] + C[k];
             }
         };
         if constexpr (L::Q == 9) collide_limrt_psi<true>(P, f, rho, U, Ft, Fi, psi, term);
@@ -833,7 +840,7 @@ __global__ void __launch_bounds__(F3_TX * F3_TY, min_blocks(F3_TX * F3_TY)) k_fu
 // never written.
 constexpr int F3_STAGES = 3;
 
-template <int F3_TX, int F3_TY, bool HAS_BC, bool EMIT>
+template <int F3_TX, int F3_TY, bool HAS_BC, bool EMIT, bool ST = false>
 __global__ void __launch_bounds__(F3_TX * F3_TY, min_blocks(F3_TX * F3_TY)) k_fused_d3q15_pipe(Params P, FusedArgs A) {
     step_dependency_wait();
     using L = D3Q15T;
@@ -943,7 +950,8 @@ __global__ void __launch_bounds__(F3_TX * F3_TY, min_blocks(F3_TX * F3_TY)) k_fu
             auto nbpsi = [&](int k) {
                 return s_psi[(z + czk<L>(k) + 3) % 3][ey + cyk<L>(k)][ex + cxk<L>(k)];
             };
-            finish_node<L, true, false, EMIT>(P, A, idc, onb, f, dum, rc, rrc, Tc, s_psi[(z + 3) % 3][ey][ex], nbpsi, 0.0);
+            finish_node<L, true, false, EMIT, decltype(nbpsi), false, ST>(P, A, idc, onb, f, dum, rc, rrc, Tc,
+                                                                          s_psi[(z + 3) % 3][ey][ex], nbpsi, 0.0);
         }
         __syncthreads();
         if (j + 2 <= z1) prefetch(j + 2);

@@ -5,6 +5,7 @@
 #pragma once
 
 #include "fused.cuh"
+#include "fused_launch.cuh"
 #include "fused_march.cuh"
 #include "fused_table.cuh"
 #include "fused_tma.cuh"
@@ -13,6 +14,11 @@
 // The marching D2Q9 step with myMRT heat (mplb_march.cu).
 int mplb_march_resident(bool f_on, bool bc);
 cudaError_t mplb_march_launch(bool f_on, bool bc, int nb, const mplb::Params& P, const mplb::FusedArgs& A, cudaStream_t s);
+
+// The general steps with a surface-tension term (mplb_st.cu).
+cudaError_t mplb_st_attributes();
+void mplb_st_launch2(int cfg, bool g_on, bool bc, int nb, const mplb::Params& P, const mplb::FusedArgs& A, cudaStream_t s);
+void mplb_st_launch3(int cfg, bool bc, int nb, const mplb::Params& P, const mplb::FusedArgs& A, cudaStream_t s);
 
 // Steps on neighbour tables (mplb_table.cu); returns the launches made.
 int mplb_table_step(int lat, int heat, bool emit, bool st, const mplb::Params& P, const mplb::TableArgs& A,
@@ -42,31 +48,14 @@ struct FusedConfig {
     TmaMapCache tmaps;
 };
 
-template <int TX, int TY, bool PIPE, bool HAS_BC, bool EMIT, bool ST = false>
-cudaError_t set_smem3() {
-    if constexpr (PIPE)
-        return cudaFuncSetAttribute(k_fused_d3q15_pipe<TX, TY, HAS_BC, EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)f3_smem<TX, TY, PIPE>());
-    else
-        return cudaFuncSetAttribute(k_fused_d3q15<TX, TY, HAS_BC, EMIT, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)f3_smem<TX, TY, PIPE>());
-}
-
 // The 3D kernels use more than the 48 KB of static shared memory.
 inline cudaError_t fused_attributes() {
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     chk(set_smem3<32, 8, false, true, true>());
     chk(set_smem3<32, 8, false, false, true>());
-    chk(set_smem3<32, 8, false, true, false, true>());
-    chk(set_smem3<32, 8, false, false, false, true>());
-#define MPLB_SET3(TX, TY, PIPE) chk(set_smem3<TX, TY, PIPE, true, false>()); chk(set_smem3<TX, TY, PIPE, false, false>());
-    MPLB_SET3(32, 8, false)
-    MPLB_SET3(32, 8, true)
-    MPLB_SET3(32, 4, false)
-    MPLB_SET3(64, 4, false)
-    MPLB_SET3(32, 16, false)
-#undef MPLB_SET3
+    chk(general_attributes<false>());
+    chk(mplb_st_attributes());
 #define MPLB_SET3_TMA(TX, TY, MINB)                                                                                          \
     chk(cudaFuncSetAttribute(k_fused_d3q15_tma<TX, TY, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,                  \
                              (int)TmaTile<TX, TY>::SMEM));                                                                  \
@@ -90,49 +79,12 @@ cudaError_t launch3_tma(FusedConfig& fc, int cfg, int nb, const Params& P, const
     return cudaSuccess;
 }
 
-template <int TX, int TY, int MINB, bool F_ON, bool G_ON, bool EMIT, bool INNER, bool MY = false, int RINGW = 0,
-          bool ST = false>
-void launch2(bool bc, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
-    constexpr int nt = TX * TY + 32 * RINGW;
-    if (bc) launch_step(k_fused_d2q9<TX, TY, MINB, F_ON, G_ON, true, EMIT, INNER, MY, RINGW, ST>, nb, nt, 0, s, P, A);
-    else launch_step(k_fused_d2q9<TX, TY, MINB, F_ON, G_ON, false, EMIT, INNER, MY, RINGW, ST>, nb, nt, 0, s, P, A);
-}
-
 // myMRT steps first fill rho_a, gsum_a (k_pullsum_d2q9).
 template <bool F_ON>
 void launch_pullsum(bool bc, const Params& P, const FusedArgs& A, cudaStream_t s) {
     const unsigned nb = (P.n + 255) / 256;
     if (bc) launch_step(k_pullsum_d2q9<F_ON, true>, nb, 256, 0, s, P, A);
     else launch_step(k_pullsum_d2q9<F_ON, false>, nb, 256, 0, s, P, A);
-}
-
-template <int TX, int TY, bool EMIT, int MINB = 0, bool INNER = false, int RINGW = 0, bool ST = false>
-void launch2_fg(bool fon, bool gon, bool bc, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
-    const bool my = gon && P.g_model == MPLB_MYMRT;
-    if (my) {
-        if constexpr (!EMIT) {
-            if (fon) launch_pullsum<true>(bc, P, A, s);
-            else launch_pullsum<false>(bc, P, A, s);
-        }
-        if (fon) launch2<TX, TY, MINB, true, true, EMIT, INNER, true, RINGW, ST>(bc, nb, P, A, s);
-        else launch2<TX, TY, MINB, false, true, EMIT, INNER, true, RINGW, false>(bc, nb, P, A, s);
-        return;
-    }
-    if (fon && gon) launch2<TX, TY, MINB, true, true, EMIT, INNER, false, RINGW, ST>(bc, nb, P, A, s);
-    else if (fon) launch2<TX, TY, MINB, true, false, EMIT, INNER, false, RINGW, ST>(bc, nb, P, A, s);
-    else if (gon) launch2<TX, TY, MINB, false, true, EMIT, INNER, false, RINGW, false>(bc, nb, P, A, s);
-}
-
-template <int TX, int TY, bool PIPE, bool EMIT, bool ST = false>
-void launch3(bool bc, int nb, const Params& P, const FusedArgs& A, cudaStream_t s) {
-    constexpr size_t sm = f3_smem<TX, TY, PIPE>();
-    if constexpr (PIPE) {
-        if (bc) launch_step(k_fused_d3q15_pipe<TX, TY, true, EMIT>, nb, TX * TY, sm, s, P, A);
-        else launch_step(k_fused_d3q15_pipe<TX, TY, false, EMIT>, nb, TX * TY, sm, s, P, A);
-    } else {
-        if (bc) launch_step(k_fused_d3q15<TX, TY, true, EMIT, ST>, nb, TX * TY, sm, s, P, A);
-        else launch_step(k_fused_d3q15<TX, TY, false, EMIT, ST>, nb, TX * TY, sm, s, P, A);
-    }
 }
 
 // Launch one fused step with candidate `cfg` (EMIT always uses candidate 0).
@@ -152,47 +104,32 @@ inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, F
         }
         cfg = fc.tile_cfg;
     }
-    // surface tension: one tile shape per kernel family stands for all candidates
-    const bool st = P.st_on && f_on && !emit;
-    const bool tma = fc.lat == MPLB_D3Q15 && CFG3[cfg].tma;
     if (fc.geom[cfg].nblocks == 0 && !emit) return cudaErrorInvalidConfiguration;  // the candidate does not take this lattice
-    if (emit || (st && !tma)) cfg = 0;
+    if (emit) cfg = 0;
     apply_geom(A, fc.geom[cfg]);
     const int nb = fc.geom[cfg].nblocks;
-    const bool bc = fc.has_bc;
+    const bool bc = fc.has_bc, st = P.st_on && f_on;
     if (fc.lat == MPLB_D2Q9) {
         if (emit) {
             launch2_fg<32, 8, true>(f_on, g_on, bc, nb, P, A, s);
-        } else if (st) {
-            launch2_fg<32, 8, false, 0, false, 0, true>(f_on, g_on, bc, nb, P, A, s);
         } else if (CFG2[cfg].march) {
             return mplb_march_launch(f_on, bc, nb, P, A, s);
         } else {
-            switch (cfg) {
-            case 0: launch2_fg<32, 8, false>(f_on, g_on, bc, nb, P, A, s); break;
-            case 1: launch2_fg<32, 4, false>(f_on, g_on, bc, nb, P, A, s); break;
-            case 2: launch2_fg<64, 4, false>(f_on, g_on, bc, nb, P, A, s); break;
-            case 3: launch2_fg<16, 8, false, 0, true>(f_on, g_on, bc, nb, P, A, s); break;
-            case 4: launch2_fg<64, 4, false, 0, true>(f_on, g_on, bc, nb, P, A, s); break;
-            case 5: launch2_fg<16, 8, false, 6, true>(f_on, g_on, bc, nb, P, A, s); break;
-            case 6: launch2_fg<32, 8, false, 3, true>(f_on, g_on, bc, nb, P, A, s); break;
-            case 7: launch2_fg<32, 4, false, 8, true>(f_on, g_on, bc, nb, P, A, s); break;
-            case 8: launch2_fg<32, 8, false, 2, false, 3>(f_on, g_on, bc, nb, P, A, s); break;
-            default: launch2_fg<16, 8, false, 4, false, 2>(f_on, g_on, bc, nb, P, A, s); break;
+            if (g_on && P.g_model == MPLB_MYMRT) {
+                if (f_on) launch_pullsum<true>(bc, P, A, s);
+                else launch_pullsum<false>(bc, P, A, s);
             }
+            if (st) mplb_st_launch2(cfg, g_on, bc, nb, P, A, s);
+            else launch_general2<false>(cfg, f_on, g_on, bc, nb, P, A, s);
         }
     } else {
         if (emit) {
             launch3<32, 8, false, true>(bc, nb, P, A, s);
-        } else if (st && !tma) {
-            launch3<32, 8, false, false, true>(bc, nb, P, A, s);
+        } else if (!CFG3[cfg].tma) {
+            if (st) mplb_st_launch3(cfg, bc, nb, P, A, s);
+            else launch_general3<false>(cfg, bc, nb, P, A, s);
         } else {
             switch (cfg) {
-            case 0: launch3<32, 8, false, false>(bc, nb, P, A, s); break;
-            case 1: launch3<32, 8, true, false>(bc, nb, P, A, s); break;
-            case 2: launch3<32, 4, false, false>(bc, nb, P, A, s); break;
-            case 3: launch3<64, 4, false, false>(bc, nb, P, A, s); break;
-            case 4: launch3<32, 16, false, false>(bc, nb, P, A, s); break;
             case 6: if (cudaError_t e = launch3_tma<32, 4, 3>(fc, cfg, nb, P, A, s)) return e; break;
             case 7: if (cudaError_t e = launch3_tma<32, 8, 2>(fc, cfg, nb, P, A, s)) return e; break;
             case 8: if (cudaError_t e = launch3_tma<32, 16, 1>(fc, cfg, nb, P, A, s)) return e; break;
@@ -466,7 +403,8 @@ inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params&
                 cudaGetLastError();
             }
         } else if (t.march) {
-            const bool my = P.g_update && model[1] == MPLB_MYMRT;
+            // (no march with a surface-tension term)
+            const bool my = P.g_update && model[1] == MPLB_MYMRT && !P.st_on;
             fc.geom[c] = my ? march_geometry(A, mplb_march_resident(P.f_update != 0, any)) : Geom{0, 0, 0, 0};
         } else {
             fc.geom[c] = fused_geometry(lat, A, t.tx, t.ty);
