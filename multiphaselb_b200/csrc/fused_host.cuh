@@ -26,6 +26,15 @@ int mplb_table_step(int lat, int heat, bool emit, bool st, const mplb::Params& P
 
 namespace mplb {
 
+// While this lives, the calling thread may allocate and wait although some other
+// stream is being captured (a step of this handle is no part of that capture,
+// and the operators, which the table kernels stand for, allocate nothing).
+struct AnyCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 struct FusedConfig {
     std::string err;
     FusedArgs args{};
@@ -39,8 +48,8 @@ struct FusedConfig {
     int ncfg = 0;
     int nblocks = 0;
     double* my_scratch = nullptr;  // myMRT: rho_a and gsum_a, 2 n doubles
-    // table candidate (D3Q15): table, flags and scratch; the
-    // best tile candidate, which takes the steps of slabs (owned and mirrored ranges)
+    // table candidate (D3Q15): table, flags and scratch (table_scratch); the best
+    // tile candidate, which takes the steps of slabs (owned and mirrored ranges)
     TableArgs tab{};
     int tile_cfg = 2;
     int* kerr = nullptr;           // kernel error flag (bounded waits), one int
@@ -87,11 +96,34 @@ void launch_pullsum(bool bc, const Params& P, const FusedArgs& A, cudaStream_t s
     else launch_step(k_pullsum_d2q9<F_ON, false>, nb, 256, 0, s, P, A);
 }
 
+// The table candidate takes steps that store every node; the others run on the
+// best tile candidate (fc.tile_cfg), as all do without its scratch.
+inline bool table_whole(const Params& P, const FusedArgs& A) { return A.own_cnt == P.n && !A.nmirror; }
+
+// That scratch, a double a node: had when the tuner times the candidate or a
+// caller forces it, given back when the tuner keeps another one.
+inline void table_scratch(FusedConfig& fc, uint32_t n, uint64_t* bytes) {
+    if (fc.tab.psi) return;
+    AnyCapture guard;
+    if (cudaMalloc((void**)&fc.tab.psi, (size_t)n * sizeof(double)) == cudaSuccess) {
+        *bytes += (size_t)n * sizeof(double);
+    } else {
+        cudaGetLastError();
+        fc.tab.psi = nullptr;
+    }
+}
+inline void table_scratch_free(FusedConfig& fc, uint32_t n, uint64_t* bytes) {
+    if (!fc.tab.psi) return;
+    cudaFree(fc.tab.psi);
+    fc.tab.psi = nullptr;
+    *bytes -= (size_t)n * sizeof(double);
+}
+
 // Launch one fused step with candidate `cfg` (EMIT always uses candidate 0).
 inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, FusedArgs A, bool f_on, bool g_on,
                                     bool emit, cudaStream_t s) {
-    if (fc.lat == MPLB_D3Q15 && CFG3[cfg].table && !emit && fc.geom[cfg].nblocks) {
-        if (A.own_cnt == P.n && !A.nmirror) {
+    if (fc.lat == MPLB_D3Q15 && CFG3[cfg].table && !emit) {
+        if (fc.tab.psi && table_whole(P, A)) {
             TableArgs T = fc.tab;
             T.fin = A.fin;
             T.fout = A.fout;
@@ -159,7 +191,7 @@ inline cudaError_t fused_launch(FusedConfig& fc, const Params& P, const FusedArg
 // follows; the heat-source history S, updated in place, is saved to `save`
 // before and restored after every candidate's launches.
 inline int fused_autotune(FusedConfig& fc, const Params& P, const FusedArgs& A, bool f_on, bool g_on, double* S,
-                          double* save, size_t n, cudaStream_t s) {
+                          double* save, size_t n, cudaStream_t s, uint64_t* bytes) {
     constexpr int SWEEPS = 3, WARM = 1, TIMED = 8;
     cudaEvent_t ev[TIMED + 1];
     int made = 0;
@@ -178,7 +210,11 @@ inline int fused_autotune(FusedConfig& fc, const Params& P, const FusedArgs& A, 
     }
     float ms_all[N_CFG_MAX][SWEEPS * TIMED];
     bool ok_c[N_CFG_MAX];
-    for (int c = 0; c < fc.ncfg; c++) ok_c[c] = fc.geom[c].nblocks > 0;
+    if (fc.lat == MPLB_D3Q15 && table_whole(P, A)) table_scratch(fc, P.n, bytes);
+    for (int c = 0; c < fc.ncfg; c++) {
+        ok_c[c] = fc.geom[c].nblocks > 0;
+        if (fc.lat == MPLB_D3Q15 && CFG3[c].table) ok_c[c] = fc.tab.psi && table_whole(P, A);
+    }
     for (int sw = 0; sw < SWEEPS; sw++) {
         for (int c = 0; c < fc.ncfg; c++) {
             bool ok = ok_c[c];
@@ -228,7 +264,9 @@ inline int fused_autotune(FusedConfig& fc, const Params& P, const FusedArgs& A, 
     fc.cfg = best_cfg;
     fc.nblocks = fc.geom[best_cfg].nblocks;
     fc.tuned = true;
-    return cudaStreamSynchronize(s) == cudaSuccess ? 0 : MPLB_E_CUDA;
+    const bool done = cudaStreamSynchronize(s) == cudaSuccess;
+    if (fc.lat == MPLB_D3Q15 && !CFG3[best_cfg].table) table_scratch_free(fc, P.n, bytes);
+    return done ? 0 : MPLB_E_CUDA;
 }
 
 // Fused path preconditions: box mesh, no serial boundary dependence, only
@@ -390,18 +428,12 @@ inline int fused_setup(FusedConfig& fc, int lat, const int* model, const Params&
             // two kernels that pull twice but have no ring, barrier or wrap arithmetic:
             // the better ones where boundary programs make a pull costly (us a step,
             // walls 97 x 61 x 83: 69 against 88 of the best tile; periodic 101 x 75 x
-            // 90: 94 against 86; B200).  Offered if the scratch, a double a node, can be had.
-            fc.geom[c] = Geom{0, 0, 0, 0};
-            if (cudaMalloc((void**)&fc.tab.psi, (size_t)n * sizeof(double)) == cudaSuccess) {
-                *bytes += (size_t)n * sizeof(double);
-                fc.tab.nb = nb;
-                fc.tab.onb = onb;
-                fc.tab.bcmap = fc.bcmap;
-                for (int q = 0; q < FUSED_MAX_PROGS; q++) fc.tab.prog[q] = A.prog[q];
-                fc.geom[c] = Geom{1, 1, 1, (int)((n + 127) / 128)};
-            } else {
-                cudaGetLastError();
-            }
+            // 90: 94 against 86; B200)
+            fc.tab.nb = nb;
+            fc.tab.onb = onb;
+            fc.tab.bcmap = fc.bcmap;
+            for (int q = 0; q < FUSED_MAX_PROGS; q++) fc.tab.prog[q] = A.prog[q];
+            fc.geom[c] = Geom{1, 1, 1, (int)((n + 127) / 128)};
         } else if (t.march) {
             // (no march with a surface-tension term)
             const bool my = P.g_update && model[1] == MPLB_MYMRT && !P.st_on;

@@ -826,13 +826,14 @@ int fused_step(mplb_gpu* h, bool emit) {
     if (!emit && !h->fc.tuned) {
         if (h->tile_request == 0) {
             RET(staging(h, h->n));
-            if (int rc = fused_autotune(h->fc, h->P, A, fon, gon, h->S, h->stage, h->n, h->stream))
+            if (int rc = fused_autotune(h->fc, h->P, A, fon, gon, h->S, h->stage, h->n, h->stream, &h->bytes))
                 return fail(rc, h->fc.err);
         } else {
             int c = h->tile_request > 0 ? h->tile_request - 1 : 0;
             if (c >= h->fc.ncfg) return fail(MPLB_E_ARG, "tile_config out of range");
             if (h->fc.geom[c].nblocks == 0)
                 return fail(MPLB_E_ARG, "tile_config " + std::to_string(h->tile_request) + " does not take this lattice");
+            if (h->lat == MPLB_D3Q15 && CFG3[c].table && table_whole(h->P, A)) table_scratch(h->fc, h->n, &h->bytes);
             h->fc.cfg = c;
             h->fc.tuned = true;
         }
@@ -995,15 +996,6 @@ int table_step(mplb_gpu* h, bool emit) {
     }
     return 0;
 }
-
-// While this lives, the calling thread may allocate and wait although some other
-// stream is being captured (a step of this handle is no part of that capture,
-// and the operators, which the table kernels stand for, allocate nothing).
-struct AnyCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~AnyCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
 
 // Enter the fused state.  Without memory for the kernels' buffers the lattice
 // stays on the operators.
