@@ -68,7 +68,10 @@ namespace {
 
 thread_local std::string g_err = "";
 
+// An error that the runtime keeps for cudaGetLastError is reported once, here;
+// the next call's launch check would take it for its own.
 int fail(int code, const std::string& msg) {
+    if (code == MPLB_E_CUDA) cudaGetLastError();
     g_err = msg;
     return code;
 }
