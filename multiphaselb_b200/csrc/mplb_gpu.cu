@@ -1295,6 +1295,7 @@ int mplb_gpu_create(const mplb_mesh_desc* mesh, const mplb_eos_desc* eos, const 
     int rc = 0;
     auto bail = [&](int code) {
         std::string keep = g_err;
+        fused_free(h->fc);
         free_all(h);
         if (h->own_stream) cudaStreamDestroy(h->stream);
         delete h;

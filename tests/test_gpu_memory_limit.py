@@ -4,6 +4,7 @@ import gc
 import pytest
 
 from multiphaselb_b200 import abi, cases
+from tests.helpers import mymrt
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +42,27 @@ def test_call_after_a_failed_create(gpu_lib):
         lat.initialize()
         lat.step(2)
         lat.download()
+
+
+def test_failed_create_gives_everything_back(gpu_lib):
+    """A myMRT column of 2 Mi nodes needs 478 bytes a node.  With less, its create
+    fails at one allocation or another, and leaves the device as it was."""
+    import torch
+    from multiphaselb_b200 import Lattice, MplbError
+    c = cases.column_case(1024, 2048)
+    c.g = mymrt(abi.D2Q9, [abi.BC_FIXEDT] * 2, c.g["bc_value"])
+    with Lattice(c, path=abi.PATH_FUSED):  # what a create loads is on the device from here on
+        pass
+    failed = 0
+    for per_node in range(400, 500, 8):
+        with Nearly(per_node * c.n):
+            left = []
+            for _ in range(3):
+                try:
+                    Lattice(c, path=abi.PATH_FUSED).close()
+                except MplbError as e:
+                    assert e.code == abi.E_CUDA
+                    failed += 1
+                left.append(torch.cuda.mem_get_info()[0])
+            assert left[0] == left[1] == left[2], (per_node, left)
+    assert 3 <= failed < 39 and failed % 3 == 0, failed
