@@ -180,10 +180,26 @@ struct mplb_gpu {
 
 namespace {
 
+bool give_back(mplb_gpu* h);
+
+// Device memory for the handle.  What it holds only to step faster goes before a
+// call fails for want of memory.
+template <class T>
+int dmalloc(mplb_gpu* h, T** p, size_t bytes) {
+    cudaError_t e = cudaMalloc((void**)p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        if (give_back(h)) e = cudaMalloc((void**)p, bytes);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    CK(e);
+    return 0;
+}
+
 template <class T>
 int dalloc(mplb_gpu* h, T** p, size_t count) {
     size_t b = std::max<size_t>(count, 1) * sizeof(T);
-    CK(cudaMalloc((void**)p, b));
+    if (int rc = dmalloc(h, p, b)) return rc;
     CK(cudaMemsetAsync(*p, 0, b, h->stream));
     h->bytes += b;
     return 0;
@@ -663,7 +679,7 @@ int staging(mplb_gpu* h, size_t elems) {
     if (h->stage) { cudaFree(h->stage); h->bytes -= h->stage_elems * sizeof(double); }
     h->stage = nullptr;
     h->stage_elems = 0;
-    CK(cudaMalloc((void**)&h->stage, elems * sizeof(double)));
+    RET(dmalloc(h, &h->stage, elems * sizeof(double)));
     h->stage_elems = elems;
     h->bytes += elems * sizeof(double);
     return 0;
@@ -1086,6 +1102,29 @@ int materialize(mplb_gpu* h) {
     else RET(fused_step(h, true));
     h->fstate = 0;
     return 0;
+}
+
+// Gives up the table kernels' buffers, if the handle has any: the operator path
+// goes back to the operators for good, the fused path to its best tile.
+bool give_back(mplb_gpu* h) {
+    if (h->path == MPLB_PATH_OPERATORS && h->tab.psi) {
+        if (materialize(h) || cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
+        h->table = false;
+        const size_t n = h->n;
+        h->bytes -= (2 * n + (h->T2 ? n : 0) + (h->U2 ? 3 * n : 0)) * sizeof(double);
+        for (double** b : {&h->tab.psi, &h->T2, &h->U2}) {
+            cudaFree(*b);
+            *b = nullptr;
+        }
+        h->tab.inv = nullptr;
+        return true;
+    }
+    if (h->path == MPLB_PATH_FUSED && h->fc.tab.psi) {
+        if (cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
+        table_scratch_free(h->fc, h->n, &h->bytes);
+        return true;
+    }
+    return false;
 }
 
 }  // namespace
@@ -1585,7 +1624,7 @@ int mplb_gpu_snapshot(mplb_gpu_t* h, int32_t flags) {
         h->snap_host = nullptr;
         h->snap_cap = 0;
         h->snap_pending = false;
-        CK(cudaMalloc((void**)&h->snap_dev, need * sizeof(double)));
+        RET(dmalloc(h, &h->snap_dev, need * sizeof(double)));
         h->bytes += need * sizeof(double);
         CK(cudaMallocHost((void**)&h->snap_host, need * sizeof(double)));
         h->snap_cap = need;
@@ -1799,7 +1838,7 @@ int mplb_gpu_run_to_equilibrium(mplb_gpu_t* h, uint32_t max_steps, uint32_t chec
         return 0;
     };
     if (fix) {
-        if (!h->mom) CK(cudaMalloc((void**)&h->mom, 6 * sizeof(long long)));
+        if (!h->mom) RET(dmalloc(h, &h->mom, 6 * sizeof(long long)));
         RET(momentum(h->mom + 3));
     }
     uint32_t done = 0;
@@ -1912,7 +1951,7 @@ int place_with_mass(mplb_gpu* h, const std::function<int(double)>& place_at, dou
         w = (fa == fb) ? 0.0 : fa / (fa - fb);
     }
     double* tmp = nullptr;
-    CK(cudaMalloc((void**)&tmp, (size_t)h->n * sizeof(double)));
+    RET(dmalloc(h, &tmp, (size_t)h->n * sizeof(double)));
     auto blend = [&]() -> int {
         RET(g_at(ra, &fa));
         CK(cudaMemcpyAsync(tmp, h->rho, (size_t)h->n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));

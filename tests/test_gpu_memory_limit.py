@@ -1,9 +1,10 @@
 """Lattices on a nearly full device: what a failed call leaves behind."""
 import gc
 
+import numpy as np
 import pytest
 
-from multiphaselb_b200 import abi, cases
+from multiphaselb_b200 import abi, cases, mesh
 from tests.helpers import mymrt
 
 pytestmark = pytest.mark.gpu
@@ -66,3 +67,60 @@ def test_failed_create_gives_everything_back(gpu_lib):
                 left.append(torch.cuda.mem_get_info()[0])
             assert left[0] == left[1] == left[2], (per_node, left)
     assert 3 <= failed < 39 and failed % 3 == 0, failed
+
+
+def channel(nx, ny):
+    """A thermal channel around a disc: no box, so the operator path."""
+    m = mesh.channel_with_cylinder(nx, ny, nx / 2 - 0.5, ny / 2.5, ny / 5.0)
+    col = cases.column_case(nx, ny)
+    keep = np.array([x + nx * y for x, y, _ in m.points.tolist()])
+    tc = col.meta["Tc"]
+    f = dict(col.f, bc_type=[abi.BC_BOUNCEBACK] * 3, bc_value=np.zeros((3, 3)))
+    g = dict(col.g, bc_type=[abi.BC_FIXEDT] * 3, bc_value=np.array([[0.86 * tc, 0, 0], [0.84 * tc, 0, 0], [0.87 * tc, 0, 0]]))
+    return mesh.mesh_case(m, "channel", col.eos, f, g, col.rho[keep], col.U[keep], col.T[keep],
+                          meta=dict(Tc=tc, box=False))
+
+
+def walls3d():
+    c = cases.bubble_case(abi.D3Q15, 16, 4.0, 3.0, 0.75, dims=(193, 121, 167))
+    c.nb, c.points, c.patches, c.patch_names = cases.box_mesh(abi.D3Q15, c.dims, (False, True, False))
+    c.periodic = (False, True, False)
+    c.f = dict(c.f, bc_type=[abi.BC_BOUNCEBACK] * len(c.patches), bc_value=np.zeros((len(c.patches), 3)))
+    return cases.perturbed(c, du=1e-3)
+
+
+# bytes a node left once the lattice has stepped: the snapshot of all fields needs
+# 8 (6 + 2 Q), 192 and 288; the table kernels' buffers are 48 and 8
+@pytest.mark.parametrize("make,kw,left", [(lambda: channel(1024, 768), dict(path=abi.PATH_OPERATORS), 170),
+                                          (walls3d, dict(path=abi.PATH_FUSED, tile_config=6), 284)])
+def test_table_buffers_go_before_a_call_fails(gpu_lib, make, kw, left):
+    """A snapshot that fits only without the table kernels' buffers is taken, and
+    the steps after it go on as if nothing had happened."""
+    import torch
+    from multiphaselb_b200 import Lattice
+    case = make()
+
+    def run(limit):
+        with Lattice(case, **kw) as lat:
+            lat.upload_case()
+            lat.initialize()
+            lat.step(3)
+            lat.sync()
+            held = lat.info()["device_bytes"]
+            if limit:
+                with Nearly(left * case.n):
+                    lat.snapshot(pdfs=True)
+                    snap = lat.snapshot_wait()
+            else:
+                lat.snapshot(pdfs=True)
+                snap = lat.snapshot_wait()
+            assert (lat.info()["device_bytes"] < held + 8 * case.n * (6 + 2 * case.Q)) == limit
+            lat.step(3)
+            torch.cuda.synchronize()
+            return snap, lat.download()
+
+    (want_snap, want), (snap, got) = run(False), run(True)
+    for k in want_snap:
+        assert np.array_equal(snap[k], want_snap[k]), k
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
