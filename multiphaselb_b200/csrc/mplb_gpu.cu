@@ -1634,10 +1634,11 @@ int mplb_gpu_snapshot(mplb_gpu_t* h, int32_t flags) {
         CK(cudaEventCreateWithFlags(&h->snap_ready, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&h->snap_done, cudaEventDisableTiming));
     }
-    // the device copy must not be rewritten while the previous one is in flight
-    if (h->snap_pending) CK(cudaStreamWaitEvent(h->stream, h->snap_done, 0));
+    // the rebuild of the reference state overlaps the previous snapshot's transfer;
+    // the device copy must not be rewritten while that is in flight
     RET(materialize(h));
     if (with_p) RET(DISPATCH(h, op_pressure, h));
+    if (h->snap_pending) CK(cudaStreamWaitEvent(h->stream, h->snap_done, 0));
     CK(cudaMemcpyAsync(h->snap_dev, h->rho, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->snap_dev + n, h->T, n * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
     if (with_p)
