@@ -119,9 +119,11 @@ inline void table_scratch_free(FusedConfig& fc, uint32_t n, uint64_t* bytes) {
     *bytes -= (size_t)n * sizeof(double);
 }
 
-// Launch one fused step with candidate `cfg` (EMIT always uses candidate 0).
+// Launch one fused step with candidate `cfg` (EMIT always uses candidate 0);
+// *launches: the kernels that takes.
 inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, FusedArgs A, bool f_on, bool g_on,
-                                    bool emit, cudaStream_t s) {
+                                    bool emit, cudaStream_t s, int* launches) {
+    *launches = 1;
     if (fc.lat == MPLB_D3Q15 && CFG3[cfg].table && !emit) {
         if (fc.tab.psi && table_whole(P, A)) {
             TableArgs T = fc.tab;
@@ -131,7 +133,7 @@ inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, F
             T.Uold = A.Uold;
             T.Unew = A.Unew;
             T.rho = A.rho_out;  // rewritten with the reference state
-            mplb_table_step(fc.lat, TABLE_NONE, false, P.st_on != 0, P, T, s);
+            *launches = mplb_table_step(fc.lat, TABLE_NONE, false, P.st_on != 0, P, T, s);
             return cudaGetLastError();
         }
         cfg = fc.tile_cfg;
@@ -148,6 +150,7 @@ inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, F
             return mplb_march_launch(f_on, bc, nb, P, A, s);
         } else {
             if (g_on && P.g_model == MPLB_MYMRT) {
+                *launches = 2;
                 if (f_on) launch_pullsum<true>(bc, P, A, s);
                 else launch_pullsum<false>(bc, P, A, s);
             }
@@ -172,10 +175,9 @@ inline cudaError_t fused_launch_cfg(FusedConfig& fc, int cfg, const Params& P, F
     return cudaGetLastError();
 }
 
-inline cudaError_t fused_launch(FusedConfig& fc, const Params& P, const FusedArgs& A, int lat, bool f_on,
-                                bool g_on, bool emit, cudaStream_t s) {
-    (void)lat;
-    return fused_launch_cfg(fc, fc.cfg, P, A, f_on, g_on, emit, s);
+inline cudaError_t fused_launch(FusedConfig& fc, const Params& P, const FusedArgs& A, bool f_on, bool g_on, bool emit,
+                                cudaStream_t s, int* launches) {
+    return fused_launch_cfg(fc, fc.cfg, P, A, f_on, g_on, emit, s, launches);
 }
 
 // Time every candidate on the current state and keep the fastest.  Three
@@ -220,7 +222,8 @@ inline int fused_autotune(FusedConfig& fc, const Params& P, const FusedArgs& A, 
             bool ok = ok_c[c];
             for (int r = 0; r < WARM + TIMED && ok; r++) {
                 if (r >= WARM) cudaEventRecord(ev[r - WARM], s);
-                ok = fused_launch_cfg(fc, c, P, A, f_on, g_on, false, s) == cudaSuccess;
+                int launches;
+                ok = fused_launch_cfg(fc, c, P, A, f_on, g_on, false, s, &launches) == cudaSuccess;
             }
             if (ok) cudaEventRecord(ev[TIMED], s);
             if (ok && cudaEventSynchronize(ev[TIMED]) == cudaSuccess) {

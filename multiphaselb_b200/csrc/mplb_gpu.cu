@@ -857,8 +857,9 @@ int fused_step(mplb_gpu* h, bool emit) {
             h->fc.tuned = true;
         }
     }
-    cudaError_t e = fused_launch(h->fc, h->P, A, h->lat, fon, gon, emit, h->stream);
-    h->launches++;
+    int launches = 0;
+    cudaError_t e = fused_launch(h->fc, h->P, A, fon, gon, emit, h->stream, &launches);
+    h->launches += launches;
     if (e != cudaSuccess) return fail(MPLB_E_CUDA, std::string("fused kernel launch: ") + cudaGetErrorString(e));
     if (!emit && h->nmirror) RET(mirror_order_after(h));
     if (!emit) {
