@@ -594,7 +594,8 @@ class FusedSlabRun:
     plane away and, for the psi / 1/rho / T / U ring of its tile, the pull
     sources of the ring one plane further: so the halo holds two planes of
     the fused state (post-collision populations, T and U of the last step),
-    copied from the neighbouring slabs' owned planes before every step
+    three with myMRT heat (T_n of a ring node holds its heat source, which
+    takes 1/rho_n one plane further out), copied from the neighbouring slabs' owned planes before every step
     (mplb_gpu_copy_state, two copies per cut and direction).  The kernel also
     updates the halo planes; what it writes there is never read before the
     next exchange overwrites it.  The owned planes are then bit-identical to
@@ -609,13 +610,11 @@ class FusedSlabRun:
     the first and last slab).
     """
 
-    HALO = 2
-
     def __init__(self, case: Case, nslabs: int, device: int = -1, stream=None, tile_config: int = 0,
                  mirror: bool = False):
         """mirror=True: the step kernels write the halo themselves
         (mplb_gpu_set_owned, mplb_gpu_add_mirror): every slab stores its owned
-        nodes only and also stores its two planes next to each cut into the
+        nodes only and also stores its planes next to each cut into the
         neighbour's next-step input, so a step is one kernel per slab and no
         copies; the halo is exchanged with copies only before the first step
         and after a gather (which brings the handles back to the reference's
@@ -623,7 +622,8 @@ class FusedSlabRun:
         from . import Lattice, PATH_FUSED
         self.case, self.nslabs = case, nslabs
         self.nplanes, self.plane, self.periodic = _box_geometry(case)
-        self.slabs = fused_slab_parts(case, nslabs, self.HALO)
+        self.halo = 3 if case.g is not None and case.g["model"] == abi.MYMRT and case.g["update"] else 2
+        self.slabs = fused_slab_parts(case, nslabs, self.halo)
         self.mirror = mirror
         self._primed = False
         for s in self.slabs:
@@ -637,7 +637,7 @@ class FusedSlabRun:
     def exchanges(self):
         """(destination slab, destination node, source slab, source node, nodes)
         of every halo copy of a step."""
-        return halo_copies(self.slabs, self.nslabs, self.plane, self.HALO)
+        return halo_copies(self.slabs, self.nslabs, self.plane, self.halo)
 
     def initialize(self):
         for s in self.slabs:
