@@ -601,9 +601,10 @@ __device__ __forceinline__ void fused2_tile(const Params& P, const FusedArgs& A,
         if constexpr (INNER) pull_node_inner<L, F_ON, G_ON>(P, A, id, f, g, rho, T);
         else pull_node<L, F_ON, G_ON, HAS_BC>(P, A, x, y, 0, id, f, g, rho, T);
         if constexpr (MY) {
-            // myMRTTemperature.c:22-31: T_n = sum g'' + S_n / 2
+            // myMRTTemperature.c:22-31: T_n = sum g'' + S_n / 2.  The rebuild takes the T_n
+            // that the step stored: a slab's halo holds its neighbour's T_n, but not its S_n.
             if constexpr (EMIT) {
-                T = T + 0.5 * A.S[id];
+                T = A.Tnew[id];
             } else {
                 s_own = heat_my<INNER>(P, A, x, y, id);
                 T = T + 0.5 * s_own;

@@ -829,7 +829,7 @@ int fused_step(mplb_gpu* h, bool emit) {
     }
     const bool udb = fon && gon;  // U double-buffered (the heat source reads U_{n-1})
     A.Told = gon ? (emit ? h->T2 : h->T) : h->T;
-    A.Tnew = gon ? h->T2 : nullptr;
+    A.Tnew = gon ? (emit ? h->T : h->T2) : nullptr;
     A.Uold = udb ? (emit ? h->U2 : h->U) : h->U;
     A.Unew = udb ? (emit ? h->U : h->U2) : h->U;
     A.S = h->S;
