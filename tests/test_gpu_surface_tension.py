@@ -4,6 +4,7 @@ the oracle; and a forced candidate runs the kernel of its own tile."""
 import pytest
 
 from multiphaselb_b200 import abi, cases
+from tests.captured import captured_kernels
 from tests.helpers import (assert_same, cylinder_d2q9, mymrt, run_checker, surface_tension_d2q9, surface_tension_d3q15)
 
 pytestmark = pytest.mark.gpu
@@ -50,7 +51,8 @@ def test_every_candidate(gpu_lib, name):
     tiles = TILES2 if case.lattice == abi.D2Q9 else TILES3
     ran = []
     for c, tile in tiles.items():
-        with Lattice(case, path=abi.PATH_FUSED, tile_config=c) as lat:
+        stream = torch.cuda.Stream()
+        with Lattice(case, path=abi.PATH_FUSED, tile_config=c, stream=stream.cuda_stream) as lat:
             lat.upload_case()
             lat.initialize()
             try:
@@ -58,21 +60,19 @@ def test_every_candidate(gpu_lib, name):
             except MplbError as e:
                 assert "does not take this lattice" in str(e), e
                 continue
-            lat.sync()
-            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-                lat.step(4)
-                lat.sync()
-                torch.cuda.synchronize()
+            lat.step(4)
             assert lat.info()["tile_config"] == c - 1
             assert_same(lat.download(), want, ctx=f"{name} candidate {c - 1}")
-        names = [e.name for e in prof.events() if "k_" in e.name]
-        assert names, "no kernel seen"
+            lat.step(1)
+            lat.sync()
+            kernels = captured_kernels(stream, lambda: lat.step(2))
         if tile:
-            assert any(f"<{tile[0]}, {tile[1]}," in n.replace("(int)", "") for n in names), (c, names)
+            assert any(args[:2] == tile for _, args in kernels), (c, kernels)
+        else:
+            assert [k for k, _ in kernels] == ["k_table_sum", "k_table_finish"] * 2, kernels
         ran.append(c)
-    # the march has no surface tension; TMA tiles take the periodic box they divide
-    most = {"bubble3d": 10, "walls3d": 6}.get(name, 10)
-    assert set(ran) >= set(range(1, most + 1)) - ({9} if name == "bubble3d" and case.dims[1] % 16 else set()), ran
+    # the march has no surface tension; TMA tiles take the periodic box, which they all divide
+    assert ran == list(range(1, (6 if name == "walls3d" else 10) + 1)), ran
     with Lattice(case, path=abi.PATH_FUSED) as lat:
         lat.upload_case()
         lat.initialize()
