@@ -857,6 +857,11 @@ int fused_step(mplb_gpu* h, bool emit) {
             h->fc.tuned = true;
         }
     }
+    if (!emit && h->fc.tab.psi && !h->fc.tab_captured && h->lat == MPLB_D3Q15 && CFG3[h->fc.cfg].table) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) cudaGetLastError();
+        h->fc.tab_captured = st != cudaStreamCaptureStatusNone;
+    }
     int launches = 0;
     cudaError_t e = fused_launch(h->fc, h->P, A, fon, gon, emit, h->stream, &launches);
     h->launches += launches;
@@ -1106,7 +1111,8 @@ int materialize(mplb_gpu* h) {
 }
 
 // Gives up the table kernels' buffers, if the handle has any: the operator path
-// goes back to the operators for good, the fused path to its best tile.
+// goes back to the operators for good, the fused path to its best tile.  A scratch
+// that a caller's graph writes to when it is replayed stays until destroy.
 bool give_back(mplb_gpu* h) {
     if (h->path == MPLB_PATH_OPERATORS && h->tab.psi) {
         if (materialize(h) || cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
@@ -1120,7 +1126,7 @@ bool give_back(mplb_gpu* h) {
         h->tab.inv = nullptr;
         return true;
     }
-    if (h->path == MPLB_PATH_FUSED && h->fc.tab.psi) {
+    if (h->path == MPLB_PATH_FUSED && h->fc.tab.psi && !h->fc.tab_captured) {
         if (cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
         table_scratch_free(h->fc, h->n, &h->bytes);
         return true;

@@ -124,3 +124,39 @@ def test_table_buffers_go_before_a_call_fails(gpu_lib, make, kw, left):
         assert np.array_equal(snap[k], want_snap[k]), k
     for k in want:
         assert np.array_equal(got[k], want[k]), k
+
+
+def test_captured_table_steps_keep_their_scratch(gpu_lib):
+    """A graph of the caller's that holds steps on the table candidate writes to its
+    scratch at every replay: a call that lacks memory fails, the scratch stays."""
+    import torch
+    from multiphaselb_b200 import Lattice, MplbError
+    case = walls3d()
+    with Lattice(case, path=abi.PATH_FUSED, tile_config=6) as lat:
+        lat.upload_case()
+        lat.initialize()
+        lat.step(6)
+        want = lat.download()
+    s = torch.cuda.Stream()
+    with Lattice(case, path=abi.PATH_FUSED, tile_config=6, stream=s.cuda_stream) as lat:
+        lat.upload_case()
+        lat.initialize()
+        lat.step(2)
+        lat.sync()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            lat.step(2)
+        held = lat.info()["device_bytes"]
+        with Nearly(284 * case.n):
+            with pytest.raises(MplbError) as e:
+                lat.snapshot(pdfs=True)
+            assert e.value.code == abi.E_CUDA
+            assert lat.info()["device_bytes"] == held
+            with torch.cuda.stream(s):
+                graph.replay()
+                graph.replay()
+            torch.cuda.synchronize()
+        got = lat.download()
+        del graph
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
