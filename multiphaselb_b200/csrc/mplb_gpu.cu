@@ -1808,14 +1808,17 @@ int mplb_gpu_monitor(mplb_gpu_t* h, int32_t reset, double* max_drho, double* mas
         k_monitor_partial<float><<<parts, TPB, 0, h->stream>>>(h->n, h->Q, h->p32[0][h->cur32[0]], h->rho_ref,
                                                                h->snap, reset, h->red);
     } else {
-        // on the operator path the sum is macroDensity's, of the streamed populations
-        if (h->path == MPLB_PATH_OPERATORS) RET(materialize(h));
+        RET(table_leave_if_capturing(h));
         if (h->path == MPLB_PATH_FUSED && h->fstate == 0) {
             RET(DISPATCH(h, op_collision, h, 0));
             RET(DISPATCH(h, op_collision, h, 1));
             h->fstate = 1;
         }
-        k_monitor_partial<double><<<parts, TPB, 0, h->stream>>>(h->n, h->Q, h->F(), 0.0, h->snap, reset, h->red);
+        // on the operator path the sum is macroDensity's, of the streamed populations;
+        // after a step of the table kernels that is rho, bit for bit
+        const bool stored = h->path == MPLB_PATH_OPERATORS && h->fstate != 0;
+        k_monitor_partial<double><<<parts, TPB, 0, h->stream>>>(h->n, stored ? 1 : h->Q, stored ? h->rho : h->F(), 0.0,
+                                                                h->snap, reset, h->red);
     }
     h->launches++;
     RET(launch_check(h));
