@@ -133,6 +133,7 @@ struct mplb_gpu {
     int red_parts = 0;
     FusedConfig fc{};
     int fstate = 0;  // 0: buffers hold the reference's state; 1: post-collision (fused)
+    bool kept = false;  // fstate 1, no step since: the other buffers hold the populations before the collision
     int precision = MPLB_FP64;
     float* p32[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // FP32 deviations [field][buffer]
     int cur32[2] = {0, 0};
@@ -868,6 +869,7 @@ int fused_step(mplb_gpu* h, bool emit) {
     if (e != cudaSuccess) return fail(MPLB_E_CUDA, std::string("fused kernel launch: ") + cudaGetErrorString(e));
     if (!emit && h->nmirror) RET(mirror_order_after(h));
     if (!emit) {
+        h->kept = false;
         if (fon) h->cur[0] ^= 1;
         if (gon) {
             h->cur[1] ^= 1;
@@ -911,6 +913,7 @@ int fused32_step(mplb_gpu* h, bool emit) {
     h->launches++;
     if (e != cudaSuccess) return fail(MPLB_E_CUDA, std::string("FP32 fused kernel launch: ") + cudaGetErrorString(e));
     if (!emit) {
+        h->kept = false;
         if (fon) h->cur32[0] ^= 1;
         if (gon) {
             h->cur32[1] ^= 1;
@@ -921,10 +924,32 @@ int fused32_step(mplb_gpu* h, bool emit) {
     return 0;
 }
 
+// Before a collision that no step may follow (the rebuild takes what the last
+// step read): the populations go to the buffers that the next step writes, from
+// where materialize() takes them back.
+int keep_reference(mplb_gpu* h) {
+    for (int fi = 0; fi < 2; fi++) {
+        if (h->model[fi] == MPLB_NO_MODEL || !(fi == 0 ? h->P.f_update : h->P.g_update)) continue;
+        CK(cudaMemcpyAsync(h->pdf[fi][h->cur[fi] ^ 1], h->pdf[fi][h->cur[fi]], (size_t)h->Q * h->n * sizeof(double),
+                           cudaMemcpyDeviceToDevice, h->stream));
+    }
+    h->kept = true;
+    return 0;
+}
+int take_reference(mplb_gpu* h) {
+    for (int fi = 0; fi < 2; fi++) {
+        if (h->model[fi] == MPLB_NO_MODEL || !(fi == 0 ? h->P.f_update : h->P.g_update)) continue;
+        CK(cudaMemcpyAsync(h->pdf[fi][h->cur[fi]], h->pdf[fi][h->cur[fi] ^ 1], (size_t)h->Q * h->n * sizeof(double),
+                           cudaMemcpyDeviceToDevice, h->stream));
+    }
+    h->kept = false;
+    return 0;
+}
+
 // FP64 reference state -> FP32 post-collision deviations.  The reference
 // values are the lattice means of rho and T (any value is valid; the mean
 // keeps deviations small).
-int prologue32(mplb_gpu* h) {
+int prologue32(mplb_gpu* h, bool keep) {
     const int parts = std::min<int>(h->red_parts, (int)blocks(h->n));
     k_sum2_partial<<<parts, TPB, 0, h->stream>>>(h->n, h->rho, h->T, h->red);
     k_sum2_final<<<1, TPB, 0, h->stream>>>(parts, h->red, h->red + 2 * h->red_parts);
@@ -935,6 +960,7 @@ int prologue32(mplb_gpu* h) {
     CK(cudaStreamSynchronize(h->stream));
     h->rho_ref = r[0] / h->n;
     h->T_ref = r[1] / h->n;
+    if (keep) RET(keep_reference(h));
     RET(DISPATCH(h, op_collision, h, 0));
     RET(DISPATCH(h, op_collision, h, 1));
     FusedArgs32 B = mplb_make_args32(h->fc.args, h->P, h->rho_ref, h->T_ref);
@@ -950,9 +976,11 @@ int prologue32(mplb_gpu* h) {
 
 // Bring the buffers back to the reference's state (after the last step).
 // Enter the fused path's state (post-collision populations) from the
-// reference's: the first collision of the loop (multiPhasePP.c:163,194).
-int enter_fused(mplb_gpu* h) {
+// reference's: the first collision of the loop (multiPhasePP.c:163,194).  keep:
+// no step may follow.
+int enter_fused(mplb_gpu* h, bool keep) {
     if (h->path != MPLB_PATH_FUSED || h->precision != MPLB_FP64 || h->fstate == 1) return 0;
+    if (keep) RET(keep_reference(h));
     RET(DISPATCH(h, op_collision, h, 0));
     RET(DISPATCH(h, op_collision, h, 1));
     h->fstate = 1;
@@ -1103,7 +1131,8 @@ int table_leave_if_capturing(mplb_gpu* h) {
 int materialize(mplb_gpu* h) {
     RET(table_leave_if_capturing(h));
     if (h->fstate == 0) return 0;
-    if (h->path == MPLB_PATH_OPERATORS) RET(table_step(h, true));
+    if (h->kept) RET(take_reference(h));
+    else if (h->path == MPLB_PATH_OPERATORS) RET(table_step(h, true));
     else if (h->precision == MPLB_FP32_DEV) RET(fused32_step(h, true));
     else RET(fused_step(h, true));
     h->fstate = 0;
@@ -1516,7 +1545,7 @@ int mplb_gpu_step(mplb_gpu_t* h, uint32_t nsteps) {
     if (nsteps == 0) return 0;
     DeviceGuard guard(h->dev);
     if (h->path == MPLB_PATH_FUSED && h->precision == MPLB_FP32_DEV) {
-        if (h->fstate == 0) RET(prologue32(h));
+        if (h->fstate == 0) RET(prologue32(h, false));
         for (uint32_t s = 0; s < nsteps; s++) RET(fused32_step(h, false));
         h->current += nsteps;
         return 0;
@@ -1525,7 +1554,7 @@ int mplb_gpu_step(mplb_gpu_t* h, uint32_t nsteps) {
         if (h->nmirror && nsteps > 1)
             return fail(MPLB_E_STATE, "a handle with mirrored ranges takes one step per call (its neighbours "
                                       "step in between)");
-        RET(enter_fused(h));  // prologue: the first collision of the loop, on the reference state
+        RET(enter_fused(h, false));  // prologue: the first collision of the loop, on the reference state
         for (uint32_t s = 0; s < nsteps; s++) RET(fused_step(h, false));
         h->current += nsteps;
         return 0;
@@ -1804,16 +1833,12 @@ int mplb_gpu_monitor(mplb_gpu_t* h, int32_t reset, double* max_drho, double* mas
     const int parts = std::min<int>(h->red_parts, (int)blocks(h->n));
     double* out = h->red + 2 * (size_t)h->red_parts + 4;
     if (h->path == MPLB_PATH_FUSED && h->precision == MPLB_FP32_DEV) {
-        if (h->fstate == 0) RET(prologue32(h));
+        if (h->fstate == 0) RET(prologue32(h, true));
         k_monitor_partial<float><<<parts, TPB, 0, h->stream>>>(h->n, h->Q, h->p32[0][h->cur32[0]], h->rho_ref,
                                                                h->snap, reset, h->red);
     } else {
         RET(table_leave_if_capturing(h));
-        if (h->path == MPLB_PATH_FUSED && h->fstate == 0) {
-            RET(DISPATCH(h, op_collision, h, 0));
-            RET(DISPATCH(h, op_collision, h, 1));
-            h->fstate = 1;
-        }
+        RET(enter_fused(h, true));
         // on the operator path the sum is macroDensity's, of the streamed populations;
         // after a step of the table kernels that is rho, bit for bit
         const bool stored = h->path == MPLB_PATH_OPERATORS && h->fstate != 0;
@@ -2096,7 +2121,7 @@ int mplb_gpu_copy_state(mplb_gpu_t* dst, uint32_t dst_start, mplb_gpu_t* src, ui
     if (count == 0) return 0;
     for (mplb_gpu* h : {src, dst}) {
         DeviceGuard guard(h->dev);
-        RET(enter_fused(h));
+        RET(enter_fused(h, true));
     }
     // the input buffers of the next fused step: post-collision populations of
     // every updated field, T and U of the last step
@@ -2342,12 +2367,12 @@ void batch_free(mplb_batch* b) {
 }
 
 // Order the batch stream after every handle's queued work.
-int batch_enter(mplb_batch* b) {
+int batch_enter(mplb_batch* b, bool keep) {
     for (mplb_gpu* h : b->lat)
         if (h->stream != b->stream) CK(cudaStreamSynchronize(h->stream));
     for (mplb_gpu* h : b->lat) {
         if (h->fstate == 0) {
-            RET(prologue32(h));
+            RET(prologue32(h, keep));
             CK(cudaStreamSynchronize(h->stream));
         }
     }
@@ -2677,13 +2702,14 @@ int mplb_batch_step(mplb_batch_t* b, uint32_t nsteps) {
     if (!b) return fail(MPLB_E_ARG, "NULL batch");
     if (nsteps == 0) return 0;
     DeviceGuard guard(b->dev);
-    RET(batch_enter(b));
+    RET(batch_enter(b, false));
     const std::vector<char> all(b->lat.size(), 1);
     int nt = 0;
     RET(batch_ready(b, all, &nt));
     for (uint32_t s = 0; s < nsteps; s++) RET(batch_launch(b, b->cfg, b->grid, (int)(s & 1)));
     for (mplb_gpu* h : b->lat) {
         if (nsteps & 1) h->cur32[0] ^= 1;
+        h->kept = false;
         h->current += nsteps;
     }
     return batch_leave(b);
@@ -2694,7 +2720,7 @@ int mplb_batch_run(mplb_batch_t* b, uint32_t max_steps, uint32_t* steps_out, dou
     if (!b) return fail(MPLB_E_ARG, "NULL batch");
     DeviceGuard guard(b->dev);
     const size_t N = b->lat.size();
-    RET(batch_enter(b));
+    RET(batch_enter(b, max_steps == 0));
     std::vector<char> active(N, 1);
     std::vector<uint32_t> steps(N, 0);
     std::vector<double> rate(N, -1.0);
@@ -2749,6 +2775,7 @@ int mplb_batch_run(mplb_batch_t* b, uint32_t max_steps, uint32_t* steps_out, dou
         RET(account(b->K));
     }
     for (size_t i = 0; i < N; i++) {
+        if (steps[i]) b->lat[i]->kept = false;
         b->lat[i]->current += steps[i];
         if (steps_out) steps_out[i] = steps[i];
         if (rate_out) rate_out[i] = rate[i];
@@ -2812,13 +2839,16 @@ int mplb_batch_average(mplb_batch_t* b, uint32_t* steps_out) {
     if (steps_out) *steps_out = 0;
     if (b->win.empty()) return fail(MPLB_E_STATE, "no filter windows set (mplb_batch_filter)");
     DeviceGuard guard(b->dev);
-    RET(batch_enter(b));
+    RET(batch_enter(b, std::all_of(b->win.begin(), b->win.end(), [](uint32_t w) { return w == 0; })));
     const std::vector<char> all(b->lat.size(), 1);
     int nt = 0;
     RET(batch_ready(b, all, &nt));
     uint32_t M = 0;
     RET(batch_window(b, all, &M));
-    for (mplb_gpu* h : b->lat) h->current += M;
+    for (mplb_gpu* h : b->lat) {
+        if (M) h->kept = false;
+        h->current += M;
+    }
     if (steps_out) *steps_out = M;
     return batch_leave(b);
 }
