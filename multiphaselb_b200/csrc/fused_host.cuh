@@ -101,8 +101,8 @@ void launch_pullsum(bool bc, const Params& P, const FusedArgs& A, cudaStream_t s
 // best tile candidate (fc.tile_cfg), as all do without its scratch.
 inline bool table_whole(const Params& P, const FusedArgs& A) { return A.own_cnt == P.n && !A.nmirror; }
 
-// That scratch, a double a node: had when the tuner times the candidate or a
-// caller forces it, given back when the tuner keeps another one.
+// That scratch, a double a node: had when the tuner keeps the candidate or a
+// caller forces it.
 inline void table_scratch(FusedConfig& fc, uint32_t n, uint64_t* bytes) {
     if (fc.tab.psi) return;
     AnyCapture guard;
@@ -213,7 +213,10 @@ inline int fused_autotune(FusedConfig& fc, const Params& P, const FusedArgs& A, 
     }
     float ms_all[N_CFG_MAX][SWEEPS * TIMED];
     bool ok_c[N_CFG_MAX];
-    if (fc.lat == MPLB_D3Q15 && table_whole(P, A)) table_scratch(fc, P.n, bytes);
+    // the table candidate is timed on `save`, which these lattices do not need:
+    // an allocation that another candidate's win would undo takes 0.5 to 1 ms
+    const bool lent = fc.lat == MPLB_D3Q15 && table_whole(P, A) && !fc.tab.psi && !keep_s;
+    if (lent) fc.tab.psi = save;
     for (int c = 0; c < fc.ncfg; c++) {
         ok_c[c] = fc.geom[c].nblocks > 0;
         if (fc.lat == MPLB_D3Q15 && CFG3[c].table) ok_c[c] = fc.tab.psi && table_whole(P, A);
@@ -265,12 +268,15 @@ inline int fused_autotune(FusedConfig& fc, const Params& P, const FusedArgs& A, 
     }
     cudaGetLastError();
     for (int i = 0; i < TIMED + 1; i++) cudaEventDestroy(ev[i]);
+    if (lent) {
+        fc.tab.psi = nullptr;
+        if (CFG3[best_cfg].table) table_scratch(fc, P.n, bytes);
+        if (CFG3[best_cfg].table && !fc.tab.psi) best_cfg = fc.tile_cfg;
+    }
     fc.cfg = best_cfg;
     fc.nblocks = fc.geom[best_cfg].nblocks;
     fc.tuned = true;
-    const bool done = cudaStreamSynchronize(s) == cudaSuccess;
-    if (fc.lat == MPLB_D3Q15 && !CFG3[best_cfg].table) table_scratch_free(fc, P.n, bytes);
-    return done ? 0 : MPLB_E_CUDA;
+    return cudaStreamSynchronize(s) == cudaSuccess ? 0 : MPLB_E_CUDA;
 }
 
 // Fused path preconditions: box mesh, no serial boundary dependence, only

@@ -160,3 +160,27 @@ def test_captured_table_steps_keep_their_scratch(gpu_lib):
         del graph
     for k in want:
         assert np.array_equal(got[k], want[k]), k
+
+
+def test_tuner_needs_no_memory(gpu_lib):
+    """The tuner times the table candidate on memory that the handle has; without
+    the scratch that stepping on it takes, the lattice keeps its best tile."""
+    from multiphaselb_b200 import Lattice
+    case = walls3d()
+    with Lattice(case, path=abi.PATH_FUSED) as lat:  # also loads every kernel that the second handle runs
+        lat.upload_case()
+        lat.initialize()
+        lat.step(3)
+        want = lat.download()
+    with Lattice(case, path=abi.PATH_FUSED) as lat:
+        lat.upload_case()
+        lat.initialize()
+        held = lat.info()["device_bytes"]
+        with Nearly(4 * case.n):
+            lat.step(3)
+            info = lat.info()
+            assert info["tile_ms"][5] > 0 and info["tile_config"] != 5
+            assert info["device_bytes"] == held
+        got = lat.download()
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
