@@ -51,7 +51,6 @@ struct FusedConfig {
     // table candidate (D3Q15): table, flags and scratch (table_scratch); the best
     // tile candidate, which takes the steps of slabs (owned and mirrored ranges)
     TableArgs tab{};
-    bool tab_captured = false;  // a graph of the caller's holds steps on it: its scratch stays
     int tile_cfg = 2;
     int* kerr = nullptr;           // kernel error flag (bounded waits), one int
     int* kerr_host = nullptr;      // its pinned host copy

@@ -134,6 +134,7 @@ struct mplb_gpu {
     FusedConfig fc{};
     int fstate = 0;  // 0: buffers hold the reference's state; 1: post-collision (fused)
     bool kept = false;  // fstate 1, no step since: the other buffers hold the populations before the collision
+    bool captured = false;  // fused path: a graph of the caller's holds steps, which may run unseen at any time
     int precision = MPLB_FP64;
     float* p32[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // FP32 deviations [field][buffer]
     int cur32[2] = {0, 0};
@@ -858,11 +859,6 @@ int fused_step(mplb_gpu* h, bool emit) {
             h->fc.tuned = true;
         }
     }
-    if (!emit && h->fc.tab.psi && !h->fc.tab_captured && h->lat == MPLB_D3Q15 && CFG3[h->fc.cfg].table) {
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) cudaGetLastError();
-        h->fc.tab_captured = st != cudaStreamCaptureStatusNone;
-    }
     int launches = 0;
     cudaError_t e = fused_launch(h->fc, h->P, A, fon, gon, emit, h->stream, &launches);
     h->launches += launches;
@@ -924,10 +920,19 @@ int fused32_step(mplb_gpu* h, bool emit) {
     return 0;
 }
 
+// Steps are about to be queued on `stream`.
+void note_capture(mplb_gpu* h, cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) cudaGetLastError();
+    if (st != cudaStreamCaptureStatusNone) h->captured = true;
+}
+
 // Before a collision that no step may follow (the rebuild takes what the last
 // step read): the populations go to the buffers that the next step writes, from
-// where materialize() takes them back.
+// where materialize() takes them back.  Not with steps in a caller's graph: a
+// replay is a step that the handle does not see.
 int keep_reference(mplb_gpu* h) {
+    if (h->captured) return 0;
     for (int fi = 0; fi < 2; fi++) {
         if (h->model[fi] == MPLB_NO_MODEL || !(fi == 0 ? h->P.f_update : h->P.g_update)) continue;
         CK(cudaMemcpyAsync(h->pdf[fi][h->cur[fi] ^ 1], h->pdf[fi][h->cur[fi]], (size_t)h->Q * h->n * sizeof(double),
@@ -1155,7 +1160,7 @@ bool give_back(mplb_gpu* h) {
         h->tab.inv = nullptr;
         return true;
     }
-    if (h->path == MPLB_PATH_FUSED && h->fc.tab.psi && !h->fc.tab_captured) {
+    if (h->path == MPLB_PATH_FUSED && h->fc.tab.psi && !h->captured) {
         if (cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
         table_scratch_free(h->fc, h->n, &h->bytes);
         return true;
@@ -1544,6 +1549,8 @@ int mplb_gpu_step(mplb_gpu_t* h, uint32_t nsteps) {
     if (!h) return fail(MPLB_E_ARG, "NULL handle");
     if (nsteps == 0) return 0;
     DeviceGuard guard(h->dev);
+    // (a handle's own stream takes part in a capture only through its mirrors)
+    if (h->path == MPLB_PATH_FUSED && (!h->own_stream || h->nmirror)) note_capture(h, h->stream);
     if (h->path == MPLB_PATH_FUSED && h->precision == MPLB_FP32_DEV) {
         if (h->fstate == 0) RET(prologue32(h, false));
         for (uint32_t s = 0; s < nsteps; s++) RET(fused32_step(h, false));
@@ -2371,6 +2378,7 @@ int batch_enter(mplb_batch* b, bool keep) {
     for (mplb_gpu* h : b->lat)
         if (h->stream != b->stream) CK(cudaStreamSynchronize(h->stream));
     for (mplb_gpu* h : b->lat) {
+        if (!b->lat[0]->own_stream) note_capture(h, b->stream);
         if (h->fstate == 0) {
             RET(prologue32(h, keep));
             CK(cudaStreamSynchronize(h->stream));

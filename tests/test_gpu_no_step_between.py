@@ -70,3 +70,37 @@ def test_batch_without_steps(gpu_lib):
         same(want, lats[1].download())
     for lat in lats:
         lat.close()
+
+
+def test_monitor_before_a_replay(gpu_lib):
+    """The steps of a caller's graph run without the handle's knowledge: what they
+    leave is read, not the state before the monitor."""
+    import torch
+    from multiphaselb_b200 import Lattice
+    case = small_cases()["column_d2q9"]
+    with Lattice(case, path=abi.PATH_FUSED) as lat:
+        lat.upload_case()
+        lat.initialize()
+        lat.step(2)
+        lat.download()
+        lat.step(4)
+        want = lat.download()
+    s = torch.cuda.Stream()
+    with Lattice(case, path=abi.PATH_FUSED, stream=s.cuda_stream) as lat:
+        lat.upload_case()
+        lat.initialize()
+        lat.step(2)
+        graph = torch.cuda.CUDAGraph()
+        lat.sync()
+        with torch.cuda.graph(graph, stream=s):
+            lat.step(2)
+        lat.download()
+        lat.monitor()
+        with torch.cuda.stream(s):
+            graph.replay()
+        lat.monitor()
+        with torch.cuda.stream(s):
+            graph.replay()
+        torch.cuda.synchronize()
+        same(want, lat.download())
+        del graph
