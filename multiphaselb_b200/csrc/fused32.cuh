@@ -116,8 +116,10 @@ constexpr int axis_population(int d) {
 
 // Mass and momentum of FP32 populations in FP64: rest = mass without the axis
 // populations, axis = mass of the axis ones, mom = momentum.  The sums of
-// opposite signs share their partial sums (FP64 sums of FP32 values are exact,
-// so the grouping does not matter); each population is converted once.
+// opposite signs share their partial sums; each population is converted once.
+// The sums are exact, so that the grouping does not matter, while the values'
+// exponents span no more than 25 (24 bits each, 4 for up to 16 terms, of 53); a
+// smaller value is rounded at 2^-53 of the sum.
 template <class L>
 __device__ __forceinline__ void exact_moments(const float* f, double& rest, double& axis, double* mom) {
     double d[L::Q];
